@@ -518,8 +518,13 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         }
 
         // ---- this row of O, normalised ---------------------------------------------------------------
+        // A warp may get here one tile ahead of the slowest one, before the product of tile n-2 has even been
+        // issued; S(n-1) only vouches for the product of tile n-3, whose phase has the parity of the last one's.
+        // So both outstanding phases are waited for in turn: a wait on the last parity alone returns at once on
+        // the phase before the previous one, and the row would leave without its two last (diagonal) tiles.
         if (ok && n_tiles > 0) {
-            ok = mbar_wait_bounded(&bar_pv, (uint32_t)((n_tiles - 1) & 1));
+            if (n_tiles > 1) ok = mbar_wait_bounded(&bar_pv, (uint32_t)((n_tiles - 2) & 1));
+            ok = ok && mbar_wait_bounded(&bar_pv, (uint32_t)((n_tiles - 1) & 1));
             ok = __all_sync(DA_FULL_MASK, ok);
         }
         if (!ok) {

@@ -61,6 +61,25 @@ def test_prefill_kernel_matches_float64_softmax(da, s, hq, hk, dtype, scale):
     _close(out, _reference(q, k, v), dtype)
 
 
+def test_prefill_kernel_is_repeatable_bit_for_bit(da):
+    """The warps of a CTA may finish their last tile at different times; whatever their order, a row must hold the
+    products of all its tiles.  Many CTAs, several runs: equal bits every time."""
+    from dram_attention_b200 import _native
+    s, hq, hk = 2999, 32, 8
+    g = torch.Generator(device=DEV).manual_seed(3)
+    q, k, v = (torch.randn(s, h, 128, generator=g, device=DEV).to(torch.bfloat16) for h in (hq, hk, hk))
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    outs = []
+    for _ in range(12):
+        outs.append(torch.empty_like(q))
+        _native.check(_native.lib().da_prefill_attention(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), outs[-1].data_ptr(), s, hq, hk, 128, hq * 128, hk * 128,
+            _native.dtype_code(q.dtype), status.data_ptr(), _native.stream_ptr()))
+    torch.cuda.synchronize()
+    assert int(status) == 0
+    assert all(torch.equal(outs[0], o) for o in outs[1:])
+
+
 def test_prefill_argument_checks(da):
     from dram_attention_b200 import _native
     lib = _native.lib()
