@@ -62,6 +62,7 @@ _SIGNATURES = {
                                            c_int, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_int, c_int,
                                            c_int, c_int, c_void_p]),
     "da_decode_attention_phased_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
+    "da_decode_attention_phase1_ctas": (c_int, [c_int]),
     "da_decode_attention_phased_supported": (c_int, [c_int, c_int, c_int, c_int, c_int, c_int, c_int]),
     "da_decode_attention_phased": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                            c_void_p, c_void_p, c_longlong, c_int, c_int, c_void_p, c_int, c_void_p,

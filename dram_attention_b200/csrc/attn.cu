@@ -179,19 +179,22 @@ struct SimtMath {
     }
 };
 
-template <typename T, int D, int ROWS, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 2 : 1) decode_attention_kernel(const AttnParams p) {
+// Warps per CTA: as many as the shared memory of an SM holds stages for (float32 units are twice as large).
+template <typename M> __host__ __device__ constexpr int simt_warps() { return M::kStages * M::UNITB > 24576 ? 6 : 8; }
+
+template <typename T, int D, int ROWS>
+__global__ void __launch_bounds__(simt_warps<SimtMath<T, D, ROWS>>() * 32, 1) decode_attention_kernel(const AttnParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    decode_attention_body<SimtMath<T, D, ROWS>, WARPS, SimtMath<T, D, ROWS>::kStages>(p, smem);
+    using M = SimtMath<T, D, ROWS>;
+    decode_attention_body<M, simt_warps<M>(), M::kStages>(p, smem);
 }
 
-constexpr int kSimtPhase1Warps = 8;   // float32 stages are twice as large: 8 warps fill an SM
-
-template <typename T, int D, int ROWS, int WARPS>
-static cudaError_t launch_attn_w(const AttnParams &p, int n_kv_heads, int splits, cudaStream_t stream) {
+template <typename T, int D, int ROWS>
+static cudaError_t launch_attn(const AttnParams &p, int n_kv_heads, int splits, cudaStream_t stream) {
     using M = SimtMath<T, D, ROWS>;
+    constexpr int WARPS = simt_warps<M>();
     constexpr int SMEM = WARPS * M::kStages * M::UNITB;
-    auto kern = decode_attention_kernel<T, D, ROWS, WARPS>;
+    auto kern = decode_attention_kernel<T, D, ROWS>;
     static bool attr_set[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -208,12 +211,6 @@ static cudaError_t launch_attn_w(const AttnParams &p, int n_kv_heads, int splits
     if (p.phase != 1) return launch_dependent(kern, grid, dim3(WARPS * 32), (size_t)SMEM, stream, p);
     kern<<<grid, WARPS * 32, SMEM, stream>>>(p);
     return cudaGetLastError();
-}
-
-template <typename T, int D, int ROWS>
-static cudaError_t launch_attn(const AttnParams &p, int n_kv_heads, int splits, cudaStream_t stream) {
-    if (p.phase == 1) return launch_attn_w<T, D, ROWS, kSimtPhase1Warps>(p, n_kv_heads, splits, stream);
-    return launch_attn_w<T, D, ROWS, kAttnWarps>(p, n_kv_heads, splits, stream);
 }
 
 // float32: up to 8 query rows per launch (register budget)
@@ -310,7 +307,10 @@ static int run_attention(const AttnCall &c) {
 
     const int tokens_per_launch = max_rows_of(c.dtype) / c.rep;
     const int rows_max = (c.n_q_tokens < tokens_per_launch ? c.n_q_tokens : tokens_per_launch) * c.rep;
-    const int splits0 = attn_splits(c.n_kv_heads);
+    // the single launch: at least two units per warp, so that a short prefix does not pay for merging empty rows
+    int splits0 = attn_splits(c.n_kv_heads);
+    const int unit_splits = (c.n_prefix_tokens + c.local_capacity) / (2 * kUnitTokens * kAttnWarps) + 1;
+    if (splits0 > unit_splits) splits0 = unit_splits;
     const int part_rows = c.phase == 0 ? splits0 : c.splits1 + c.splits2;
     if (c.workspace_bytes < (size_t)kCounterBytes + partial_bytes(c.n_kv_heads, part_rows, rows_max, c.head_dim))
         return DA_ERR_WORKSPACE;
@@ -397,7 +397,7 @@ extern "C" size_t da_decode_attention_tokens_workspace_bytes(int n_kv_heads, int
     long long rows = (long long)rep * n_q_tokens;
     if (rows > da::kAttnMaxRows) rows = da::kAttnMaxRows > rep ? da::kAttnMaxRows / rep * rep : rep;
     return (size_t)da::kCounterBytes +
-           da::partial_bytes(n_kv_heads, da::attn_splits(n_kv_heads), (int)rows, head_dim);
+           da::partial_bytes(n_kv_heads, da::attn_reserved_splits(n_kv_heads), (int)rows, head_dim);
 }
 
 extern "C" size_t da_decode_attention_workspace_bytes(int n_kv_heads, int rep, int head_dim) {
@@ -499,13 +499,13 @@ extern "C" int da_decode_attention_phased_supported(int n_kv_heads, int rep, int
     if (rep > da::max_rows_of(dtype)) return 0;
     if (n_kv_heads * 4 > da::kCounterBytes) return 0;
     if (page_size % da::kUnitTokens != 0 || (long long)n_slots * page_size > 0x7fffffffLL) return 0;
-    // shared memory of a phase-1 CTA: warps x stages x stage bytes, plus the plan tables
-    const size_t esz = dtype == DA_F32 ? 4 : 2;
-    size_t stage = (size_t)da::kUnitTokens * (2 * head_dim * esz + (esz == 2 ? 16 : 0));
-    const int stages = esz == 2 ? 2 : (stage >= 16384 ? 2 : (stage >= 8192 ? 3 : 4));
-    const int warps = esz == 2 ? da::kAttnPhase1Warps : da::kSimtPhase1Warps;
-    const size_t smem = (size_t)warps * stages * stage + (size_t)warps * da::kRoundUnits * 16 + 2048;
-    return smem <= 227 * 1024 ? 1 : 0;
+    // (a float32 unit of head_dim 128 is 16 KB: an SM holds stages for six warps, too few to keep phase 1 fed)
+    if (dtype == DA_F32 && head_dim == 128) return 0;
+    return 1;
+}
+
+extern "C" int da_decode_attention_phase1_ctas(int n_kv_heads) {
+    return n_kv_heads < 1 ? 0 : phase_splits(n_kv_heads, 0, 1);
 }
 
 extern "C" size_t da_decode_attention_phased_workspace_bytes(int n_kv_heads, int rep, int head_dim) {

@@ -267,8 +267,7 @@ __device__ __forceinline__ void decode_attention_body(const AttnParams &p, unsig
 
     // ---- the CTA of this head that finished last (of both launches, when there are two) --------
     // a head that phase 2 redid: phase 1's rows (the first in the workspace) are left out
-    merge_splits<T, D, THREADS>(p, h, p.part_rows, rows, p.phase != 0 ? p.redo + h : nullptr, p.splits1, smem,
-                                WARPS * STAGES * STAGEB);
+    merge_splits<T, D, THREADS>(p, h, p.part_rows, rows, p.phase != 0 ? p.redo + h : nullptr, p.splits1, smem);
     // every CTA of this head is done with the eviction front: the one the LRU update left becomes current
     if (p.phase != 0 && tid == 0) atomicXor(p.flip + h, 1);   // (no result wanted: the CTA does not wait for it)
     if (tid == 0) p.counters[h] = 0u;

@@ -7,33 +7,37 @@
 
 namespace da {
 
-constexpr int kAttnWarps = 4;          // warps per CTA of the single launch and of phase 2
-constexpr int kAttnThreads = kAttnWarps * 32;
+constexpr int kAttnWarps = 12;         // warps per CTA (16-bit types): one CTA fills an SM
 constexpr int kUnitTokens = 16;
 constexpr int kCounterBytes = 1024;
-constexpr int kAttnTargetCtas = 444;   // 3 per SM on 148 SMs
+constexpr int kAttnSms = 148;
 constexpr int kAttnMaxSplits = 148;
 constexpr int kAttnMaxRows = 16;       // query rows (tokens x GQA group) of one KV head per launch
 constexpr int kRoundUnits = 32;        // units a warp plans at a time (one per lane)
 
-// Phase 1 runs beside the selection kernels, whose CTAs need a whole SM each.  Its CTAs are
-// therefore built to fill an SM on their own (12 warps, all of the shared memory), and by default
-// there are at most 116 of them: wherever the hardware places them, 32 of the 148 SMs stay empty.
-// Phase 2 normally covers only the few slots the LRU update could evict; 64 CTAs on those 32 SMs
-// are plenty.
-constexpr int kAttnPhase1Warps = 12;
+// CTAs per head ("splits").  Every CTA of every launch fills an SM on its own (12 warps, nearly all of the shared
+// memory): the loop of a warp is a chain of dependent instructions, so an SM wants all the warps it can hold, and one
+// large CTA leaves a third of the partial rows of three small ones to the final merge, which adds them with three
+// times the threads.  The merge ends every step: with 4-warp CTAs it took 3.2 to 5.6 us (one batch of loads is
+// a round trip of 0.9 us, and there were up to six), with 12-warp CTAs 1.9 to 2.6 us.
+//
+// Phase 1 runs beside the selection kernels, whose CTAs need a whole SM each: it has at most 116 CTAs, so that
+// wherever the hardware places them 32 of the 148 SMs stay empty.  Phase 2 covers the few slots the LRU update
+// could evict, on what phase 1 and the update's CTAs (one per head) leave.  The caps on CTAs per head keep the merge
+// at one batch per thread (4 query rows: 3 x 18 partials); the single launch also keeps at least two units per warp.
 constexpr int kAttnPhase1Ctas = 116;
-constexpr int kAttnPhase1MaxPerHead = 20;  // a shard of 1 to 4 KV heads: beyond 20 CTAs a head, every further partial
-                                           // row costs the final merge (which is on the step's critical path) more
-                                           // than the CTA adds in bandwidth (phase 1 is not on that path)
-constexpr int kAttnPhase2Ctas = 64;
-constexpr int kAttnPhase2MaxPerHead = 8;   // the front is small: more CTAs only lengthen the merge
+constexpr int kAttnPhase1MaxPerHead = 48;
+constexpr int kAttnPhase2MaxPerHead = 6;
 
 __host__ __device__ inline int attn_splits(int n_kv_heads) {
-    int s = kAttnTargetCtas / n_kv_heads;
-    if (s > kAttnMaxSplits) s = kAttnMaxSplits;
-    if (s < 1) s = 1;
-    return s;
+    const int s = kAttnSms / n_kv_heads;
+    return s < 1 ? 1 : s;
+}
+
+// what the workspace of the single launch has room for (part of the ABI; at least attn_splits)
+__host__ __device__ inline int attn_reserved_splits(int n_kv_heads) {
+    const int s = 3 * kAttnSms / n_kv_heads;
+    return s > kAttnMaxSplits ? kAttnMaxSplits : (s < 1 ? 1 : s);
 }
 
 __host__ __device__ inline int attn_splits_phase1(int n_kv_heads) {
@@ -44,7 +48,7 @@ __host__ __device__ inline int attn_splits_phase1(int n_kv_heads) {
 }
 
 __host__ __device__ inline int attn_splits_phase2(int n_kv_heads) {
-    int s = kAttnPhase2Ctas / n_kv_heads;
+    int s = (kAttnSms - n_kv_heads * (attn_splits_phase1(n_kv_heads) + 1)) / n_kv_heads;
     if (s > kAttnPhase2MaxPerHead) s = kAttnPhase2MaxPerHead;
     if (s < 1) s = 1;
     return s;
@@ -229,158 +233,133 @@ __device__ __forceinline__ int plan_commit(const AttnParams &p, const LaunchUnit
 // be read with 128-bit loads.
 template <int D> struct PartialRow { static constexpr int kWidth = D + 4; };
 
-__device__ __forceinline__ void cp_async_16(void *dst_smem, const void *src_gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst_smem)), "l"(src_gmem) : "memory");
+// Running softmax merge of (max, l, four accumulator columns); log2 domain.
+struct MergeAcc {
+    float m, l;
+    float4 a;
+};
+__device__ __forceinline__ void merge_into(MergeAcc &x, float m, float l, const float4 &v) {
+    const float mn = fmaxf(x.m, m);
+    const float ms = (mn == -INFINITY) ? 0.f : mn;
+    const float wx = fast_exp2(x.m - ms), wv = fast_exp2(m - ms);
+    x.m = mn;
+    x.l = x.l * wx + l * wv;
+    x.a.x = x.a.x * wx + v.x * wv;
+    x.a.y = x.a.y * wx + v.y * wv;
+    x.a.z = x.a.z * wx + v.z * wv;
+    x.a.w = x.a.w * wx + v.w * wv;
 }
 
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// waits until at most N of this thread's committed groups are still in flight
-template <int N> __device__ __forceinline__ void cp_async_wait_group() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
+// Final merge of the per-CTA partials of one head by one CTA of THREADS threads.  A CTA's partial = `rows` rows
+// of (acc[D] already weighted to the row's max, max, l); the partials of consecutive CTAs are contiguous in the
+// workspace.  It is on the critical path of every step and bound by latency alone, so it is one round trip to
+// L2 wherever the registers allow: a thread owns four columns of a row for every G-th CTA (G = how many
+// times the row-columns fit into the CTA), requests kMergeBatch partials together with their (max, l) pairs, and
+// folds them in registers; the G groups meet in shared memory.  (Staging the rows in shared memory in two
+// halves, as before, took one round trip per half: 3.7 us for 22 partials of 4 rows, 5.9 us for 55.)
+// `skip_flag` (may be null): when the word it points to is non-zero the first `skip` CTAs' rows are left out.
+constexpr int kMergeBatch = 18;
 
-// Final merge of the per-CTA partials of one head by one CTA of THREADS threads.  A CTA's
-// partial = `rows` rows of (acc[D] already weighted to the row's max, max, l); the partials of
-// consecutive CTAs are contiguous in the workspace.  They are brought into shared memory (the
-// idle stage buffers, `smem_bytes` of them) with 16-byte asynchronous copies that bypass L1 (the
-// rows were written by other SMs) and need no registers.  When they do not all fit, the buffer
-// is used as two halves: the next batch is on its way while the current one is added up.  The
-// first batch is requested before anything else is looked at.  `skip_flag` (may be null):
-// when the word it points to is non-zero the first `skip` CTAs' rows are left out (they get
-// weight zero); it is read together with the (max, l) pairs, so it costs no round trip.
 template <typename T, int D, int THREADS>
 __device__ __forceinline__ void merge_splits(const AttnParams &p, int h, int splits, int rows, const int32_t *skip_flag,
-                                             int skip, unsigned char *smem, int smem_bytes) {
+                                             int skip, unsigned char *smem) {
     constexpr int PW = PartialRow<D>::kWidth;
     constexpr int VPR = D / 4;          // float4 per accumulator row
-    constexpr float NEG_INF = -INFINITY;
-    constexpr int MAXE = (kAttnMaxRows * VPR + THREADS - 1) / THREADS;   // output float4 per thread
-    __shared__ float sh_m[kAttnMaxRows], sh_l[kAttnMaxRows];
     const int tid = threadIdx.x;
     const int32_t peer_step = p.peer_world > 0 ? __ldcg(p.peer_seq) : 0;   // (needed at the very end: read now)
+    const int n_skip = (skip_flag != nullptr && __ldcg(skip_flag) != 0) ? skip : 0;
     const float *hp = p.partials + ((size_t)h * p.part_rows * rows) * PW;
-    const int n = splits * rows;
-    float *wgt = reinterpret_cast<float *>(smem);   // [n] max, then weight
-    float *lsum = wgt + n;                          // [n] l of every partial row
-    const int head_bytes = ((2 * n * (int)sizeof(float)) + 15) & ~15;
-    float4 *buf0 = reinterpret_cast<float4 *>(smem + head_bytes);
-    const int cta_f4 = rows * PW / 4;               // float4 per CTA's partial
-    int chunk = (smem_bytes - head_bytes) / (cta_f4 * 16);
-    if (chunk < splits) chunk = max(chunk / 2, 1);  // two halves in flight
-    chunk = min(chunk, splits);
-    float4 *buf1 = buf0 + (size_t)chunk * cta_f4;
+    const size_t cta_stride = (size_t)rows * PW;
+    const int items = rows * VPR;
+    const int groups = max(THREADS / items, 1);
+    float4 *sh_a = reinterpret_cast<float4 *>(smem);                    // [groups - 1][items]
+    float2 *sh_ml = reinterpret_cast<float2 *>(sh_a + THREADS);         // [groups - 1][items]
+    const int g = groups > 1 ? tid / items : 0;
 
-    // one commit group per batch (also when this thread has nothing to copy in it)
-    auto request = [&](int s0, float4 *buf) {
-        const int cnt = min(chunk, splits - s0);
-        const float4 *src = reinterpret_cast<const float4 *>(hp) + (size_t)s0 * cta_f4;
-        for (int i = tid; i < cnt * cta_f4; i += THREADS) cp_async_16(buf + i, src + i);
-        cp_async_commit();
-    };
-    request(0, buf0);
-    if (chunk < splits) request(chunk, buf1);
-    const int n_skip = (skip_flag != nullptr && __ldcg(skip_flag) != 0) ? skip * rows : 0;
-    for (int i = tid; i < n; i += THREADS) {
-        const float2 ml = __ldcg(reinterpret_cast<const float2 *>(hp + (size_t)i * PW + D));
-        wgt[i] = i < n_skip ? NEG_INF : ml.x;
-        lsum[i] = ml.y;
-    }
-    __syncthreads();
-    {   // one warp per query row: common max, weights exp2(max_s - max), weighted row sum
-        const int lane = tid & 31;
-        for (int rr = tid >> 5; rr < rows; rr += THREADS / 32) {
-            float mn = NEG_INF;
-            for (int s = lane; s < splits; s += 32) mn = fmaxf(mn, wgt[s * rows + rr]);
+    for (int e0 = 0; e0 < items; e0 += THREADS) {
+        const int e = groups > 1 ? tid % items : e0 + tid;
+        const bool mine = e < items && g < groups;
+        MergeAcc x = {-INFINITY, 0.f, make_float4(0.f, 0.f, 0.f, 0.f)};
+        if (mine) {
+            const float *col = hp + (size_t)(e / VPR) * PW + 4 * (e % VPR);
+            const float *ml = hp + (size_t)(e / VPR) * PW + D;
+            for (int s0 = g; s0 < splits; s0 += groups * kMergeBatch) {
+                float4 v[kMergeBatch];
+                float2 w[kMergeBatch];
 #pragma unroll
-            for (int off = 16; off >= 1; off >>= 1) mn = fmaxf(mn, __shfl_xor_sync(DA_FULL_MASK, mn, off));
-            const float ms = (mn == NEG_INF) ? 0.f : mn;
-            float ll = 0.f;
-            for (int s = lane; s < splits; s += 32) {
-                const float w = fast_exp2(wgt[s * rows + rr] - ms);
-                wgt[s * rows + rr] = w;
-                ll = fmaf(lsum[s * rows + rr], w, ll);
-            }
+                for (int i = 0; i < kMergeBatch; ++i) {
+                    const int s = min(s0 + i * groups, splits - 1);
+                    v[i] = __ldcg(reinterpret_cast<const float4 *>(col + (size_t)s * cta_stride));
+                    w[i] = __ldcg(reinterpret_cast<const float2 *>(ml + (size_t)s * cta_stride));
+                }
+                // the batch's own maximum first, so that its exponentials do not wait for one another
+                float mb = x.m;
 #pragma unroll
-            for (int off = 16; off >= 1; off >>= 1) ll += __shfl_xor_sync(DA_FULL_MASK, ll, off);
-            if (lane == 0) {
-                sh_m[rr] = ms;
-                sh_l[rr] = ll;
-            }
-        }
-    }
-    float4 a[MAXE];
+                for (int i = 0; i < kMergeBatch; ++i) {
+                    const int s = s0 + i * groups;
+                    if (s >= splits || s < n_skip) w[i].x = -INFINITY;
+                    mb = fmaxf(mb, w[i].x);
+                }
+                const float ms = (mb == -INFINITY) ? 0.f : mb;
+                const float wx = fast_exp2(x.m - ms);
+                x.m = mb;
+                x.l *= wx;
+                x.a.x *= wx; x.a.y *= wx; x.a.z *= wx; x.a.w *= wx;
 #pragma unroll
-    for (int k = 0; k < MAXE; ++k) a[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    int which = 0;
-    for (int s0 = 0; s0 < splits; s0 += chunk, which ^= 1) {
-        const int cnt = min(chunk, splits - s0);
-        const float4 *buf = which ? buf1 : buf0;
-        if (s0 + chunk < splits) cp_async_wait_group<1>(); else cp_async_wait_group<0>();   // this batch has landed
-        __syncthreads();      // the batch and (first time round) the weights are in shared memory
-#pragma unroll
-        for (int k = 0; k < MAXE; ++k) {
-            const int e = k * THREADS + tid;
-            if (e < rows * VPR) {
-                const int r = e / VPR, c4 = e % VPR;
-                const float4 *col = buf + r * (PW / 4) + c4;
-                for (int s = 0; s < cnt; ++s) {
-                    const float4 v = col[s * cta_f4];
-                    const float w = wgt[(s0 + s) * rows + r];
-                    a[k].x = fmaf(v.x, w, a[k].x);
-                    a[k].y = fmaf(v.y, w, a[k].y);
-                    a[k].z = fmaf(v.z, w, a[k].z);
-                    a[k].w = fmaf(v.w, w, a[k].w);
+                for (int i = 0; i < kMergeBatch; ++i) {
+                    if (w[i].x == -INFINITY) continue;   // (a CTA without units: its rows are zeros)
+                    const float wv = fast_exp2(w[i].x - ms);
+                    x.l = fmaf(w[i].y, wv, x.l);
+                    x.a.x = fmaf(v[i].x, wv, x.a.x);
+                    x.a.y = fmaf(v[i].y, wv, x.a.y);
+                    x.a.z = fmaf(v[i].z, wv, x.a.z);
+                    x.a.w = fmaf(v[i].w, wv, x.a.w);
                 }
             }
         }
-        if (s0 + 2 * chunk < splits) {
-            __syncthreads();  // everybody is done with this half: the batch after the next goes into it
-            request(s0 + 2 * chunk, which ? buf1 : buf0);
+        if (groups > 1) {
+            if (mine && g > 0) {
+                sh_a[(g - 1) * items + e] = x.a;
+                sh_ml[(g - 1) * items + e] = make_float2(x.m, x.l);
+            }
+            __syncthreads();
+            if (mine && g == 0) {
+                for (int k = 0; k < groups - 1; ++k) {
+                    const float2 w = sh_ml[k * items + e];
+                    merge_into(x, w.x, w.y, sh_a[k * items + e]);
+                }
+            }
         }
-    }
-#pragma unroll
-    for (int k = 0; k < MAXE; ++k) {
-        const int e = k * THREADS + tid;
-        if (e < rows * VPR) {
+        if (mine && g == 0) {
             const int r = e / VPR, c4 = e % VPR;
-            const float ll = sh_l[r];
-            const float inv = ll > 0.f ? 1.f / ll : 0.f;
+            const float inv = x.l > 0.f ? 1.f / x.l : 0.f;
             // row r = (query token, head of the group)
             const int tok = p.q_tok0 + r / p.rep;
             const size_t orow = (size_t)tok * p.n_kv_heads * p.rep + (size_t)h * p.rep + r % p.rep;
+            union { T t[4]; uint32_t w[sizeof(T)]; } o;   // four elements as whole words (2 or 4 of them)
+            o.t[0] = from_float<T>(x.a.x * inv);
+            o.t[1] = from_float<T>(x.a.y * inv);
+            o.t[2] = from_float<T>(x.a.z * inv);
+            o.t[3] = from_float<T>(x.a.w * inv);
             T *dst = reinterpret_cast<T *>(p.out) + orow * D + 4 * c4;
-            const T v0 = from_float<T>(a[k].x * inv), v1 = from_float<T>(a[k].y * inv),
-                    v2 = from_float<T>(a[k].z * inv), v3 = from_float<T>(a[k].w * inv);
-            dst[0] = v0;
-            dst[1] = v1;
-            dst[2] = v2;
-            dst[3] = v3;
-            if (c4 == 0 && p.lse_out) p.lse_out[orow] = (sh_m[r] + log2f(ll)) * 0.6931471805599453f;
+            if constexpr (sizeof(T) == 4) *reinterpret_cast<uint4 *>(dst) = make_uint4(o.w[0], o.w[1], o.w[2], o.w[3]);
+            else *reinterpret_cast<uint2 *>(dst) = make_uint2(o.w[0], o.w[1]);
+            if (c4 == 0 && p.lse_out)
+                p.lse_out[orow] = ((x.m == -INFINITY ? 0.f : x.m) + log2f(x.l)) * 0.6931471805599453f;
             if (p.peer_world > 0) {
                 // these four values as payload words {payload, tag} into slot (seq & 1) of every rank's buffer,
                 // at this rank's place (one query token per call: orow is the head row)
                 const int32_t sq = peer_step;
                 const uint32_t tag = (uint32_t)(sq + 1);
-                constexpr int NW = (int)(4 * sizeof(T) / 4);
-                uint32_t w[NW];
-                if constexpr (sizeof(T) == 4) {
-                    w[0] = __float_as_uint((float)v0);
-                    w[1] = __float_as_uint((float)v1);
-                    w[NW - 2] = __float_as_uint((float)v2);
-                    w[NW - 1] = __float_as_uint((float)v3);
-                } else {
-                    auto bits = [](T v) -> uint32_t { return (uint32_t)(*reinterpret_cast<const unsigned short *>(&v)); };
-                    w[0] = bits(v0) | (bits(v1) << 16);
-                    w[NW - 1] = bits(v2) | (bits(v3) << 16);
-                }
+                constexpr int NW = (int)sizeof(T);
                 const size_t word0 = (size_t)(sq & 1) * p.peer_world * p.peer_words + (size_t)p.peer_rank * p.peer_words +
                                      (orow * D + 4 * c4) * sizeof(T) / 4;
 #pragma unroll
-                for (int g = 0; g < kAttnMaxPeers; ++g) {
-                    if (g < p.peer_world) {
-                        uint2 *pd = p.peer_buf[g] + word0;
+                for (int gp = 0; gp < kAttnMaxPeers; ++gp) {
+                    if (gp < p.peer_world) {
+                        uint2 *pd = p.peer_buf[gp] + word0;
 #pragma unroll
-                        for (int i = 0; i < NW; ++i) st_word_sys(pd + i, w[i], tag);
+                        for (int i = 0; i < NW; ++i) st_word_sys(pd + i, o.w[i], tag);
                     }
                 }
             }

@@ -241,18 +241,19 @@ struct MmaMath {
     }
 };
 
-// WARPS per CTA, STAGES per warp, at least MINB CTAs per SM.
-template <typename T, int D, bool FULL, int WARPS, int STAGES, int MINB>
-__global__ void __launch_bounds__(WARPS * 32, MINB) decode_attention_mma_kernel(const AttnParams p) {
+constexpr int kMmaStages = 2;   // per warp: 12 x 2 stages are 203 KB of an SM's shared memory for head_dim 128
+
+template <typename T, int D, bool FULL>
+__global__ void __launch_bounds__(kAttnWarps * 32, 1) decode_attention_mma_kernel(const AttnParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    decode_attention_body<MmaMath<T, D, FULL>, WARPS, STAGES>(p, smem);
+    decode_attention_body<MmaMath<T, D, FULL>, kAttnWarps, kMmaStages>(p, smem);
 }
 
-template <typename T, int D, bool FULL, int WARPS, int STAGES, int MINB>
-static cudaError_t launch_mma_w(const AttnParams &p, int n_kv_heads, int splits, cudaStream_t stream) {
+template <typename T, int D, bool FULL>
+static cudaError_t launch_mma(const AttnParams &p, int n_kv_heads, int splits, cudaStream_t stream) {
     using M = MmaMath<T, D, FULL>;
-    constexpr int SMEM = WARPS * STAGES * M::STAGEB;
-    auto kern = decode_attention_mma_kernel<T, D, FULL, WARPS, STAGES, MINB>;
+    constexpr int SMEM = kAttnWarps * kMmaStages * M::STAGEB;
+    auto kern = decode_attention_mma_kernel<T, D, FULL>;
     static bool attr_set[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -266,19 +267,9 @@ static cudaError_t launch_mma_w(const AttnParams &p, int n_kv_heads, int splits,
     dim3 grid(splits, n_kv_heads);
     // phase 1 runs on a stream of its own beside the kernels of the step; the other launches follow
     // the LRU update in their stream and may move onto the SMs while it is still running
-    if (p.phase != 1) return launch_dependent(kern, grid, dim3(WARPS * 32), (size_t)SMEM, stream, p);
-    kern<<<grid, WARPS * 32, SMEM, stream>>>(p);
+    if (p.phase != 1) return launch_dependent(kern, grid, dim3(kAttnWarps * 32), (size_t)SMEM, stream, p);
+    kern<<<grid, kAttnWarps * 32, SMEM, stream>>>(p);
     return cudaGetLastError();
-}
-
-// Geometry.  The loop of a warp is a chain of dependent instructions (wait, ldmatrix, mma,
-// softmax, issue), so an SM needs many warps to keep its copies flowing: 12 warps with two
-// stages each (203 KB of stages per SM for head_dim 128).  The single launch and phase 2 use
-// three 4-warp CTAs per SM; phase 1 one 12-warp CTA that fills its SM.
-template <typename T, int D, bool FULL>
-static cudaError_t launch_mma(const AttnParams &p, int n_kv_heads, int splits, cudaStream_t stream) {
-    if (p.phase == 1) return launch_mma_w<T, D, FULL, kAttnPhase1Warps, 2, 1>(p, n_kv_heads, splits, stream);
-    return launch_mma_w<T, D, FULL, kAttnWarps, 2, 3>(p, n_kv_heads, splits, stream);
 }
 
 template <typename T, int D>

@@ -269,8 +269,8 @@ class DRAMAttention(torch.nn.Module):
         # Only inside a graph capture: a graph dispatches the scorer's CTAs ahead of phase 1's (node
         # order), whereas two eager launches that become ready together (a backlogged GPU) may be
         # dispatched either way round, and phase 1 first would starve the scorer of SMs.
-        budget = self.selection_sm_budget or max(
-            1, 148 - self.n_kv_heads * (self.phase1_ctas or min(20, max(1, 116 // self.n_kv_heads))))
+        budget = self.selection_sm_budget or max(1, 148 - self.n_kv_heads * (
+            self.phase1_ctas or _native.lib().da_decode_attention_phase1_ctas(self.n_kv_heads)))
         early = self.fork_before_score and torch.cuda.is_current_stream_capturing()
         if early:
             self._fork.record(main)

@@ -371,12 +371,14 @@ DA_API int da_decode_attention_fetch(const void *q,
  * split_order, split_count, split_flip, split_redo   the evict_queue, front_count, split_flip and
  *            split_redo of da_lru_update (called with split_advance = 0 between the two launches).
  * phase1_ctas, phase2_ctas  CTAs per KV head of the two launches, the same values in both
- *            calls of a step; 0 = defaults (116 / n_kv_heads and 64 / n_kv_heads), at most 148.
+ *            calls of a step; 0 = defaults (phase 1: da_decode_attention_phase1_ctas(); phase 2: what
+ *            that and one CTA per head of the update leave of 148), at most 148.
  * workspace  da_decode_attention_phased_workspace_bytes() bytes, shared by both phases.
  */
 DA_API size_t da_decode_attention_phased_workspace_bytes(int n_kv_heads, int rep, int head_dim);
-/* 1 if da_decode_attention_phased accepts this shape (page_size a multiple of 16, the phase-1
- * CTA fits an SM's shared memory), else 0. */
+/* Default CTAs per KV head of phase 1; each fills an SM (for the sm_budget of da_topk_pages_wide). */
+DA_API int da_decode_attention_phase1_ctas(int n_kv_heads);
+/* 1 if da_decode_attention_phased accepts this shape (page_size a multiple of 16), else 0. */
 DA_API int da_decode_attention_phased_supported(int n_kv_heads, int rep, int head_dim, int dtype,
                         int n_slots, int page_size, int local_capacity);
 DA_API int da_decode_attention_phased(int phase, const int32_t *split_order, const int32_t *split_count,

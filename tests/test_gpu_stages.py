@@ -481,6 +481,18 @@ def test_decode_attention_matches_oracle(da, dtype, d, hk, rep, n_prefix, cap, t
     _attention_case(da, dtype, d, hk, rep, n_prefix, cap, t_new, n_prefix + t_new, device_pos)
 
 
+@pytest.mark.parametrize("dtype,d,hk,rep,n_prefix,cap,t_new", [
+    (torch.bfloat16, 128, 1, 16, 60000, 40, 20),     # 148 partials, more row-columns than threads, many batches
+    (torch.bfloat16, 64, 1, 1, 60000, 40, 20),       # one row of 64 channels: 24 groups of threads
+    (torch.bfloat16, 128, 7, 3, 3000, 40, 20),       # a group count that does not divide the CTA
+    (torch.float32, 128, 1, 8, 20000, 40, 20),       # six-warp CTAs
+    (torch.float16, 128, 40, 2, 800, 40, 20),        # three partials per head
+    (torch.bfloat16, 128, 160, 4, 48, 40, 20),       # more heads than SMs: one partial, nothing to add
+])
+def test_final_merge_of_the_partials(da, dtype, d, hk, rep, n_prefix, cap, t_new):
+    _attention_case(da, dtype, d, hk, rep, n_prefix, cap, t_new, n_prefix + hk, False)
+
+
 @pytest.mark.parametrize("dtype,d,hk,rep,n_prefix,cap,t0,s_q", [
     (torch.bfloat16, 128, 2, 4, 512, 96, 40, 2),     # 8 rows: the half-tile kernel
     (torch.bfloat16, 128, 2, 4, 512, 96, 40, 4),     # 16 rows: the full tile
