@@ -6,6 +6,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 from ctypes import c_char_p, c_float, c_int, c_int32, c_longlong, c_size_t, c_void_p, POINTER
 
 import torch
@@ -73,6 +74,9 @@ _SIGNATURES = {
     "da_decode_attention_static": (c_int, [c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_longlong,
                                            c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p,
                                            c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
+    "da_generate": (c_int, [c_char_p]),
+    "da_fork_create": (c_int, [POINTER(c_void_p)]),
+    "da_fork_destroy": (None, [c_void_p]),
     "da_build_pages": (c_int, [c_void_p, c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p,
                                c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
 }
@@ -97,6 +101,37 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+# layouts and argument block of da_generate: every field 8 bytes, in the header's order
+LAYOUT_RESIDENT, LAYOUT_FETCH_KERNEL, LAYOUT_FETCH_IN_ATTENTION, LAYOUT_OVERLAPPED = 0, 1, 2, 3
+_GENERATE_FIELDS = 59
+_PACK = struct.Struct(f"={_GENERATE_FIELDS}q").pack
+
+
+def generate(*fields: int) -> None:
+    """da_generate with the fields of da_generate_args in order; missing trailing ones are 0."""
+    code = lib().da_generate(_PACK(*fields, *(0,) * (_GENERATE_FIELDS - len(fields))))
+    if code != 0:
+        check(code, "da_generate")
+
+
+class Fork:
+    """Side stream and events of the two-launch layout, on the device current at construction."""
+
+    def __init__(self):
+        self.handle = None
+        out = c_void_p()
+        check(lib().da_fork_create(ctypes.byref(out)), "da_fork_create")
+        self.handle, self._destroy = out.value, lib().da_fork_destroy
+
+    def __deepcopy__(self, memo):
+        return Fork()
+
+    def __del__(self):
+        if self.handle:
+            self._destroy(self.handle)
+            self.handle = None
+
+
 def check(code: int, what: str = "") -> None:
     if code != 0:
         text = lib().da_error_string(code).decode()
@@ -111,8 +146,8 @@ def dtype_code(dtype: torch.dtype) -> int:
 
 
 def stream_ptr() -> int:
-    """cudaStream_t of torch's current stream."""
-    return torch.cuda.current_stream().cuda_stream
+    """cudaStream_t of torch's current stream on the current device."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def status_message(bits: int) -> str:

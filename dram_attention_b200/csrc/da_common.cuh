@@ -157,6 +157,10 @@ static inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, 
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// The scorer behind da_score_pages; `started` (may be null) is recorded when all its CTAs have begun.
+int score_pages(const void *q, const void *summaries, float *scores, int n_tokens, int n_kv_heads, int rep, int n_pages,
+                int head_dim, int dtype, int summaries_ordered, cudaStream_t stream, cudaEvent_t started);
+
 // ---- peer gather words ---------------------------------------------------------------
 // The all-gather of the head shards moves 8-byte words {4 bytes of payload, the step's tag}: one naturally
 // aligned 8-byte store per word arrives whole, so a word that carries the tag carries its payload.

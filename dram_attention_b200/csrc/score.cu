@@ -20,6 +20,25 @@ constexpr int kScoreThreads = 256;
 constexpr int kScoreWarps = kScoreThreads / 32;
 constexpr int kScoreUnroll = 4;
 
+// `started` (may be null) is recorded when every CTA of the launch has begun: a launch on another stream that
+// waits for it gets the SMs as this kernel's CTAs leave them, and never ahead of them.
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_scorer(void (*kernel)(KArgs...), dim3 grid, cudaStream_t stream, cudaEvent_t started, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kScoreThreads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    if (started) {
+        attr[0].id = cudaLaunchAttributeLaunchCompletionEvent;
+        attr[0].val.launchCompletionEvent.event = started;
+        attr[0].val.launchCompletionEvent.flags = 0;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 template <typename T, int VEC, int REP>
 __global__ void __launch_bounds__(kScoreThreads, 2)
 score_pages_kernel(const T *__restrict__ q, const T *__restrict__ summaries, float *__restrict__ scores,
@@ -261,7 +280,7 @@ score_pages_mma_kernel(const T *__restrict__ q, const T *__restrict__ summaries,
 
 template <typename T, int D>
 static cudaError_t launch_mma(const void *q, const void *summaries, float *scores, int n_tokens, int n_kv_heads,
-                              int rep, int n_pages, cudaStream_t stream) {
+                              int rep, int n_pages, cudaStream_t stream, cudaEvent_t started) {
     int per_row = kScoreMmaCtasPerHeadTarget / (n_kv_heads * n_tokens);
     if (per_row < 1) per_row = 1;
     const int n_tiles = (n_pages + 7) / 8;
@@ -271,18 +290,17 @@ static cudaError_t launch_mma(const void *q, const void *summaries, float *score
     const T *qq = static_cast<const T *>(q);
     const T *ss = static_cast<const T *>(summaries);
     switch (rep) {
-    case 1: score_pages_mma_kernel<T, D, 1><<<grid, kScoreThreads, 0, stream>>>(qq, ss, scores, n_kv_heads, n_pages); break;
-    case 2: score_pages_mma_kernel<T, D, 2><<<grid, kScoreThreads, 0, stream>>>(qq, ss, scores, n_kv_heads, n_pages); break;
-    case 4: score_pages_mma_kernel<T, D, 4><<<grid, kScoreThreads, 0, stream>>>(qq, ss, scores, n_kv_heads, n_pages); break;
-    case 8: score_pages_mma_kernel<T, D, 8><<<grid, kScoreThreads, 0, stream>>>(qq, ss, scores, n_kv_heads, n_pages); break;
+    case 1: return launch_scorer(score_pages_mma_kernel<T, D, 1>, grid, stream, started, qq, ss, scores, n_kv_heads, n_pages);
+    case 2: return launch_scorer(score_pages_mma_kernel<T, D, 2>, grid, stream, started, qq, ss, scores, n_kv_heads, n_pages);
+    case 4: return launch_scorer(score_pages_mma_kernel<T, D, 4>, grid, stream, started, qq, ss, scores, n_kv_heads, n_pages);
+    case 8: return launch_scorer(score_pages_mma_kernel<T, D, 8>, grid, stream, started, qq, ss, scores, n_kv_heads, n_pages);
     default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 template <typename T, int VEC>
 static cudaError_t launch_fast(const void *q, const void *summaries, float *scores, int n_tokens,
-                               int n_kv_heads, int rep, int n_pages, cudaStream_t stream) {
+                               int n_kv_heads, int rep, int n_pages, cudaStream_t stream, cudaEvent_t started) {
     const int n_pairs = (n_pages + 1) / 2;
     // two resident CTAs per SM; spread them over the heads and tokens of the launch
     int per_row = (148 * 2) / (n_kv_heads * n_tokens);
@@ -294,41 +312,55 @@ static cudaError_t launch_fast(const void *q, const void *summaries, float *scor
     const T *qq = static_cast<const T *>(q);
     const T *ss = static_cast<const T *>(summaries);
     switch (rep) {
-    case 1: score_pages_kernel<T, VEC, 1><<<grid, kScoreThreads, 0, stream>>>(qq, ss, scores, n_kv_heads, n_pages); break;
-    case 2: score_pages_kernel<T, VEC, 2><<<grid, kScoreThreads, 0, stream>>>(qq, ss, scores, n_kv_heads, n_pages); break;
-    case 4: score_pages_kernel<T, VEC, 4><<<grid, kScoreThreads, 0, stream>>>(qq, ss, scores, n_kv_heads, n_pages); break;
+    case 1: return launch_scorer(score_pages_kernel<T, VEC, 1>, grid, stream, started, qq, ss, scores, n_kv_heads, n_pages);
+    case 2: return launch_scorer(score_pages_kernel<T, VEC, 2>, grid, stream, started, qq, ss, scores, n_kv_heads, n_pages);
+    case 4: return launch_scorer(score_pages_kernel<T, VEC, 4>, grid, stream, started, qq, ss, scores, n_kv_heads, n_pages);
     default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 template <typename T>
 static cudaError_t launch_generic(const void *q, const void *summaries, float *scores, int n_tokens,
-                                  int n_kv_heads, int rep, int n_pages, int head_dim, cudaStream_t stream) {
+                                  int n_kv_heads, int rep, int n_pages, int head_dim,
+                                  cudaStream_t stream, cudaEvent_t started) {
     int gx = (n_pages + kScoreWarps - 1) / kScoreWarps;
     if (gx > 592) gx = 592;
     dim3 grid(gx, n_kv_heads, n_tokens);
-    score_pages_generic_kernel<T><<<grid, kScoreThreads, 0, stream>>>(
-        static_cast<const T *>(q), static_cast<const T *>(summaries), scores, n_kv_heads, rep, n_pages, head_dim);
-    return cudaGetLastError();
+    return launch_scorer(score_pages_generic_kernel<T>, grid, stream, started, static_cast<const T *>(q),
+                         static_cast<const T *>(summaries), scores, n_kv_heads, rep, n_pages, head_dim);
 }
 
 template <typename T>
 static cudaError_t dispatch(const void *q, const void *summaries, float *scores, int n_tokens, int n_kv_heads,
-                            int rep, int n_pages, int head_dim, bool ordered, cudaStream_t stream) {
+                            int rep, int n_pages, int head_dim, bool ordered, cudaStream_t stream, cudaEvent_t started) {
     const bool aligned = (((uintptr_t)q | (uintptr_t)summaries) & 15) == 0;
     if constexpr (sizeof(T) == 2) {
         if (ordered && aligned && (rep == 1 || rep == 2 || rep == 4 || rep == 8)) {
-            if (head_dim == 128) return launch_mma<T, 128>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, stream);
-            if (head_dim == 64) return launch_mma<T, 64>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, stream);
+            if (head_dim == 128) return launch_mma<T, 128>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, stream, started);
+            if (head_dim == 64) return launch_mma<T, 64>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, stream, started);
         }
     }
     const bool rep_ok = rep == 1 || rep == 2 || rep == 4;
     if (aligned && rep_ok) {
-        if (head_dim == 128) return launch_fast<T, 8>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, stream);
-        if (head_dim == 64) return launch_fast<T, 4>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, stream);
+        if (head_dim == 128) return launch_fast<T, 8>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, stream, started);
+        if (head_dim == 64) return launch_fast<T, 4>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, stream, started);
     }
-    return launch_generic<T>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, head_dim, stream);
+    return launch_generic<T>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, head_dim, stream, started);
+}
+
+int score_pages(const void *q, const void *summaries, float *scores, int n_tokens, int n_kv_heads, int rep,
+                int n_pages, int head_dim, int dtype, int summaries_ordered, cudaStream_t s, cudaEvent_t started) {
+    if (!q || !summaries || !scores) return DA_ERR_NULL;
+    if (n_tokens < 1 || n_kv_heads < 1 || rep < 1 || n_pages < 1 || head_dim < 1) return DA_ERR_SHAPE;
+    if (n_kv_heads > 65535 || n_tokens > 65535) return DA_ERR_UNSUPPORTED;
+    cudaError_t e;
+    switch (dtype) {
+    case DA_F32: e = dispatch<float>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, head_dim, summaries_ordered != 0, s, started); break;
+    case DA_F16: e = dispatch<__half>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, head_dim, summaries_ordered != 0, s, started); break;
+    case DA_BF16: e = dispatch<__nv_bfloat16>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, head_dim, summaries_ordered != 0, s, started); break;
+    default: return DA_ERR_DTYPE;
+    }
+    return (int)e;
 }
 
 }  // namespace da
@@ -336,18 +368,8 @@ static cudaError_t dispatch(const void *q, const void *summaries, float *scores,
 extern "C" int da_score_pages(const void *q, const void *summaries, float *scores, int n_tokens,
                               int n_kv_heads, int rep, int n_pages, int head_dim, int dtype,
                               int summaries_ordered, da_stream_t stream) {
-    if (!q || !summaries || !scores) return DA_ERR_NULL;
-    if (n_tokens < 1 || n_kv_heads < 1 || rep < 1 || n_pages < 1 || head_dim < 1) return DA_ERR_SHAPE;
-    if (n_kv_heads > 65535 || n_tokens > 65535) return DA_ERR_UNSUPPORTED;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    cudaError_t e;
-    switch (dtype) {
-    case DA_F32: e = da::dispatch<float>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, head_dim, summaries_ordered != 0, s); break;
-    case DA_F16: e = da::dispatch<__half>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, head_dim, summaries_ordered != 0, s); break;
-    case DA_BF16: e = da::dispatch<__nv_bfloat16>(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, head_dim, summaries_ordered != 0, s); break;
-    default: return DA_ERR_DTYPE;
-    }
-    return (int)e;
+    return da::score_pages(q, summaries, scores, n_tokens, n_kv_heads, rep, n_pages, head_dim, dtype,
+                           summaries_ordered, static_cast<cudaStream_t>(stream), nullptr);
 }
 
 DA_DEFINE_TRACE_SETTER(trace_set_score)

@@ -61,6 +61,7 @@ class DRAMAttention(torch.nn.Module):
         self._can_overlap = False
         self._overlap_ok = {}
         self._side = None
+        self._fork_handle = None
         self._prefill_status = None
 
     # stage="prefill": this package's tcgen05 kernel where it applies (16-bit, head_dim 128)
@@ -70,8 +71,10 @@ class DRAMAttention(torch.nn.Module):
     # front) runs on a side stream beside scoring, selection and LRU update; the second (the few
     # slots of the front, with the miss fetch) follows the update without waiting for the first.
     overlap = True
-    # ... and, when the step is being captured into a CUDA graph, that first launch forks off before
-    # the page scorer rather than after it
+    # ... and that first launch starts once every CTA of the page scorer has begun, taking over the SMs as they
+    # leave them, rather than after the scorer.  (Waiting for the scorer's start, not merely being enqueued
+    # behind it, is what keeps a graph from dispatching it first: it then left the scorer 32 of 148 SMs and a
+    # 128K layer took 60 us instead of 40.)
     fork_before_score = True
     # CTAs per KV head of the two launches (0: the library's defaults)
     phase1_ctas = 0
@@ -223,27 +226,76 @@ class DRAMAttention(torch.nn.Module):
         xq = xq if xq.is_contiguous() else xq.contiguous()
         xk = xk if xk.is_contiguous() else xk.contiguous()
         xv = xv if xv.is_contiguous() else xv.contiguous()
-        with torch.cuda.device(xq.device):
-            out = torch.empty_like(xq)
-            if seqlen > 1:
-                # several tokens: one scoring / selection / LRU update over all of them (list of
-                # seqlen * rep * k pages per KV head), the gather-copy of the misses, then the
-                # attention of every token over the same slot table
-                self.lru_cache.get_kv_cache_(xq)
-                self.attend_(xq, xk, xv, start_pos, out)
-            elif self._can_overlap and self.fused_fetch and self.overlap and self._overlap_supported(rep, xq.dtype):
-                self._generate_overlapped(xq, xk, xv, start_pos, out)
-            elif self._can_fuse and self.fused_fetch:
-                # score -> select -> LRU update -> attention that also brings in the misses
-                lc = self.lru_cache
-                _, page_list = lc.top_k_selector.page_list_(xq, lc.top_k)
-                lc.update_tables_(page_list, inline_fetch=True, after_selection=True)
-                self.attend_(xq, xk, xv, start_pos, out, fetch=True)
-            else:
-                # score -> select -> LRU update -> fetch (no-ops for a fully resident prefix)
-                self.lru_cache.get_kv_cache_(xq)
-                self.attend_(xq, xk, xv, start_pos, out)
+        if xq.device.index != torch.cuda.current_device():
+            with torch.cuda.device(xq.device):
+                return self._enqueue_generate(xq, xk, xv, start_pos, seqlen, rep)
+        return self._enqueue_generate(xq, xk, xv, start_pos, seqlen, rep)
+
+    def _enqueue_generate(self, xq, xk, xv, start_pos, seqlen: int, rep: int):
+        """The launches of a generate call on the current stream.  Layouts: a resident prefix needs the attention
+        only; several tokens per call take one scoring / selection / LRU update over all of them (a list of
+        seqlen * rep * k pages per KV head), the gather-copy of the misses, then the attention of every
+        token over the same slot table; one token takes the two-launch layout where it applies."""
+        lc = self.lru_cache
+        out = torch.empty_like(xq)
+        if isinstance(lc, DummyCache):
+            layout = _native.LAYOUT_RESIDENT
+        elif seqlen > 1 or not (self._can_fuse and self.fused_fetch):
+            layout = _native.LAYOUT_FETCH_KERNEL
+        elif self._can_overlap and self.overlap and self._overlap_supported(rep, xq.dtype):
+            layout = _native.LAYOUT_OVERLAPPED
+        else:
+            layout = _native.LAYOUT_FETCH_IN_ATTENTION
+        if layout != _native.LAYOUT_RESIDENT and not lc.updates_natively():
+            self._generate_stage_by_stage(layout, xq, xk, xv, start_pos, out)
+            return out
+        if isinstance(start_pos, torch.Tensor):
+            assert start_pos.dtype == torch.int32 and start_pos.is_cuda and start_pos.numel() == 1
+            pos_dev, pos_host = start_pos.data_ptr(), 0
+        else:
+            pos_dev, pos_host = 0, int(start_pos)
+        buf, nbytes, status = self._workspace(rep, xq.device, seqlen)
+        own = self._buffers
+        cache_k, cache_v = own["cache_k"], own["cache_v"]
+        hk, dtype = self.n_kv_heads, _native.dtype_code(xq.dtype)
+        _, tok_stride, head_stride, _ = cache_k.stride()
+        if layout == _native.LAYOUT_RESIDENT:
+            if lc.num_tokens == 0:
+                raise RuntimeError("empty DRAM prefix is not supported")
+            slots, cache_fields = lc.hbm_kv_cache, ()
+            table = (slots.data_ptr(), slots.stride(0), lc.num_tokens, 0, 0)
+        else:
+            table, cache_fields = lc.generate_fields(seqlen, rep, xq.dtype, self.selection_sm_budget)
+        fork = 0
+        if layout == _native.LAYOUT_OVERLAPPED:
+            if self._fork_handle is None:
+                self._fork_handle = _native.Fork()
+            fork = self._fork_handle.handle
+        push = self.peer_push
+        if push is not None and seqlen == 1:
+            cache_fields = cache_fields or LRUCache.NO_GENERATE_FIELDS
+            cache_fields += (push[0].value, push[1], push[2], push[3], push[4])
+        _native.generate(
+            layout, _native.stream_ptr(), fork, int(self.fork_before_score),
+            xq.data_ptr(), xk.data_ptr(), xv.data_ptr(), out.data_ptr(), pos_dev, pos_host, seqlen,
+            hk, rep, self.head_dim, dtype, *table, cache_k.data_ptr(), cache_v.data_ptr(), tok_stride, head_stride,
+            cache_k.shape[1], self.dram_kv_cache_size, buf.data_ptr(), nbytes, status.data_ptr(),
+            int(self.phase1_ctas), int(self.phase2_ctas), *cache_fields)
         return out
+
+    def _generate_stage_by_stage(self, layout: int, xq, xk, xv, start_pos, out) -> None:
+        """The same launches through the classes' own methods, for a cache whose update_tables_ was replaced."""
+        lc = self.lru_cache
+        if layout == _native.LAYOUT_OVERLAPPED:
+            self._generate_overlapped(xq, xk, xv, start_pos, out)
+        elif layout == _native.LAYOUT_FETCH_IN_ATTENTION:
+            # score -> select -> LRU update -> attention that also brings in the misses
+            _, page_list = lc.top_k_selector.page_list_(xq, lc.top_k)
+            lc.update_tables_(page_list, inline_fetch=True, after_selection=True)
+            self.attend_(xq, xk, xv, start_pos, out, fetch=True)
+        else:
+            lc.get_kv_cache_(xq)
+            self.attend_(xq, xk, xv, start_pos, out)
 
     def _overlap_supported(self, rep: int, dtype) -> bool:
         ok = self._overlap_ok.get(rep)

@@ -216,6 +216,33 @@ class LRUCache(torch.nn.Module):
             int(self.inline_fetch_max) if inline_fetch else 0,
             self.status.data_ptr(), _native.stream_ptr()), "da_lru_update")
 
+    def updates_natively(self) -> bool:
+        """Whether a generate call may enqueue the update itself instead of calling update_tables_ (it may not
+        when a subclass or the instance replaced that method)."""
+        return type(self).update_tables_ is LRUCache.update_tables_ and "update_tables_" not in self.__dict__
+
+    NO_GENERATE_FIELDS = (0,) * 23
+
+    def generate_fields(self, seq_len: int, rep: int, dtype: torch.dtype, selection_sm_budget: int):
+        """The slot table's and the cache's fields of _native.generate, read afresh for every call."""
+        b = self._buffers
+        sel = self.top_k_selector
+        k = min(self.top_k, sel.num_pages)
+        assert sel.chunk_min_max.dtype == b["hbm_kv_cache"].dtype == dtype, "query dtype must match the key summaries"
+        scores, page_list = sel._workspace(seq_len, rep, k)
+        miss_pages, miss_slots, n_miss = self._miss_buffers(seq_len * rep * k)
+        slots, dram = b["hbm_kv_cache"], b["dram_kv_cache"]
+        table = (slots.data_ptr(), slots.stride(0), self.num_hbm_pages * self.page_size, self.num_hbm_pages,
+                 self.page_size)
+        cache = (sel.chunk_min_max.data_ptr(), scores.data_ptr(), page_list.data_ptr(), self.num_dram_pages, k,
+                 int(selection_sm_budget), dram.data_ptr(), b["dram_page_to_hbm_page_mapping"].data_ptr(),
+                 b["hbm_page_to_dram_page_mapping"].data_ptr(), b["page_access_time"].data_ptr(),
+                 b["step_counters"].data_ptr(), miss_pages.data_ptr(), miss_slots.data_ptr(), n_miss.data_ptr(),
+                 b["slot_source"].data_ptr(), b["evict_order"].data_ptr(), b["n_evictable"].data_ptr(),
+                 b["evict_flip"].data_ptr(), b["evict_redo"].data_ptr(), int(self.split_cap),
+                 dram.shape[2] * dram.element_size(), int(self.inline_fetch_max), b["status"].data_ptr())
+        return table, cache
+
     def fetch_(self, list_len: int) -> None:
         """Enqueue the gather-copy of the pages the last update_tables_ found missing."""
         miss_pages, miss_slots, n_miss = self._miss_buffers(list_len)

@@ -540,6 +540,75 @@ DA_API int da_gather_heads(const void *local, int bytes_per_rank, void *const *p
                     int32_t *seq, int rank, int world, void *out, int timeout_us, int32_t *status,
                     da_stream_t stream);
 
+/*
+ * A whole generate call: everything DRAMAttention._generate enqueues (dram_attention/dram_attention.py:144-177),
+ * as one library call.  The other entry points stay for callers that keep the reference's classes and swap
+ * single kernels.
+ *
+ * da_generate_args: every field is 8 bytes (pointer or int64), so that a caller without a C compiler can pack it.
+ * The fields mean what the parameters of the same name of the single entry points mean.
+ *   layout   DA_LAYOUT_RESIDENT            the whole prefix is in `slots` (n_prefix_tokens of them): attention only
+ *            DA_LAYOUT_FETCH_KERNEL        score, select, update, da_fetch_pages, attention; any n_q_tokens
+ *            DA_LAYOUT_FETCH_IN_ATTENTION  score, select, update, da_decode_attention_fetch; one token
+ *            DA_LAYOUT_OVERLAPPED          the two-launch attention: phase 1 on the fork's stream beside score,
+ *                                          select and update, phase 2 after the update; one token
+ *   fork     from da_fork_create (one per concurrent caller); needed by DA_LAYOUT_OVERLAPPED
+ *   fork_before_score   non-zero: phase 1 starts once every CTA of the scorer has begun, so that it takes over
+ *            the SMs as they leave them; zero: after the scorer
+ *   selection_sm_budget   0: 148 minus phase 1's CTAs
+ *   peer_buffers (may be null), peer_seq, peer_rank, peer_world, peer_bytes   as da_decode_attention_push_next
+ * Scores, page list and the miss list are scratch of the caller, sized for n_q_tokens.  The call works inside a stream
+ * capture.  The fork's stream is joined to `stream` before the call returns.
+ */
+#define DA_LAYOUT_RESIDENT 0
+#define DA_LAYOUT_FETCH_KERNEL 1
+#define DA_LAYOUT_FETCH_IN_ATTENTION 2
+#define DA_LAYOUT_OVERLAPPED 3
+
+typedef struct da_generate_args {
+    int64_t layout;
+    da_stream_t stream;
+    void *fork;
+    int64_t fork_before_score;
+    /* this call */
+    const void *q, *new_k, *new_v;
+    void *out;
+    const int32_t *start_pos_dev;
+    int64_t start_pos_host, n_q_tokens;
+    /* shape */
+    int64_t n_kv_heads, rep, head_dim, dtype;
+    /* attention */
+    void *slots;
+    int64_t slots_head_stride, n_prefix_tokens, n_slots, page_size;
+    void *local_k, *local_v;
+    int64_t local_token_stride, local_head_stride, local_capacity, dram_tokens;
+    void *workspace;
+    int64_t workspace_bytes;
+    int32_t *status;
+    int64_t phase1_ctas, phase2_ctas;
+    /* selection (not read by DA_LAYOUT_RESIDENT, nor is anything below up to the peers) */
+    const void *summaries;
+    float *scores;
+    int32_t *page_list;
+    int64_t n_dram_pages, top_k, selection_sm_budget;
+    /* LRU update and fetch */
+    const void *dram_pages;
+    int32_t *dram_to_slot, *slot_to_dram, *access_time, *step, *miss_pages, *miss_slots, *n_miss, *slot_source;
+    int32_t *evict_queue, *front_count, *split_flip, *split_redo;
+    int64_t split_cap, page_bytes, inline_fetch_max;
+    int32_t *lru_status;
+    /* head sharding */
+    void *const *peer_buffers;
+    const int32_t *peer_seq;
+    int64_t peer_rank, peer_world, peer_bytes;
+} da_generate_args;
+
+DA_API int da_generate(const da_generate_args *args);
+
+/* The side stream and events of DA_LAYOUT_OVERLAPPED, on the current device (host objects; no device memory). */
+DA_API int da_fork_create(void **fork);
+DA_API void da_fork_destroy(void *fork);
+
 #ifdef __cplusplus
 }
 #endif

@@ -676,3 +676,32 @@ def test_single_kv_head_shard(da):
     """One GPU's share at 8-way KV-head sharding of the 128K layer: one KV head, four query heads."""
     w = llama_layer_workload(seed=0, steps=3, n_kv_heads=1)
     _check_layer_invariants(da, w, 3)
+
+
+@pytest.mark.parametrize("layout,counts", [((True, True), [1, 1, 1]), ((True, False), [1, 1, 1]), ((False, False), [1, 1, 1]),
+                                           ((True, True), [3, 1, 2])])
+def test_one_library_call_equals_stage_by_stage(da, layout, counts):
+    """A generate call enqueued by the library in one go against the same call made through the classes'
+    methods (which a replaced update_tables_ selects): same outputs and tables to the bit."""
+    w = llama_layer_workload(seed=11, steps=8, dram_tokens=8192, n_kv_heads=2, lru=4096, local=256, top_k=512,
+                             redraw_every=2)
+    ms = []
+    for staged in (False, True):
+        m = da.DRAMAttention(device=DEV, dtype=torch.bfloat16, **w.ctor_kwargs())
+        m.init_cache(w.k.to(DEV), w.v.to(DEV))
+        m.fused_fetch, m.overlap = layout
+        if staged:
+            m.lru_cache.update_tables_ = m.lru_cache.update_tables_
+        assert m.lru_cache.updates_natively() != staged
+        ms.append(m)
+    pos = w.prefill_len
+    for i, n in enumerate(counts):
+        ins = [t[i:i + n, 0, 0][None].to(DEV) for t in (w.xq, w.xk, w.xv)]
+        a, b = (m(*ins, start_pos=pos, stage="generate") for m in ms)
+        assert torch.equal(a, b)
+        pos += n
+    for name in ("hbm_kv_cache", "page_access_time", "hbm_page_to_dram_page_mapping", "slot_source", "evict_redo"):
+        assert torch.equal(getattr(ms[0].lru_cache, name), getattr(ms[1].lru_cache, name)), name
+    assert torch.equal(ms[0].cache_k, ms[1].cache_k)
+    for m in ms:
+        m.check_status()
