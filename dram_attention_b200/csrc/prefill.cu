@@ -2,41 +2,37 @@
 // head_dim 128, on the 5th-generation tensor cores: tcgen05.mma with both operands in shared
 // memory (filled by TMA tensor copies, 128-byte swizzle) and the accumulators in tensor memory.
 //
-// One CTA per (128 query rows, query head), TWO CTAs per SM: four softmax warps and one issuing
-// warp each.  Softmax thread t owns query row t, which is lane t of tensor memory, so the
-// softmax needs no shuffles: a row's logits come back with tcgen05.ld as plain registers of
-// its thread.  One lane of the fifth warp issues every MMA, one lane of the sixth every TMA
+// One CTA per (128 query rows, query head), TWO CTAs per SM.  Eight softmax warps: a query row is a lane of tensor
+// memory and has two threads, in warps w and w + 4, one per half of a tile's keys; they tell each other their
+// maxima through shared memory, and otherwise a row's logits come back with tcgen05.ld as plain registers of a
+// thread, without shuffles.  One lane of the ninth warp issues every MMA, one lane of the tenth every TMA
 // copy; the roles meet only at mbarriers (tile arrived, S ready, P ready, product complete),
-// never at a CTA-wide barrier.  The MMA lane's instruction stream sets the pace of the CTA
-// (measured with time stamps: 1.4 us per tile when it also issued the copies and rebuilt its
-// operand descriptors per MMA), hence a warp of its own and descriptors made before the loop.
-// A CTA alone leaves the tensor core idle most of the time: its softmax is a chain of phases
-// (read S, maximum, exponentials on the special-function unit, sum, conversion, write P) that
-// the same four warps walk tile after tile.  Two CTAs on an SM walk it out of step, so one's
-// exponentials overlap the other's loads, conversions and hand-offs, and both feed the tensor
-// core.  To fit twice, a CTA takes 64-key tiles (97 KB of shared memory) and 256 columns of
-// tensor memory.  Per 64-key tile:
+// never at a CTA-wide barrier.  Per 128-key tile:
 //
-//   S = Q K^T      8 MMAs (M128 N64 K16), Q and the key tile K-major          -> TMEM columns 0..63 / 64..127
+//   S = Q K^T      8 MMAs (M128 N128 K16), Q and the key tile K-major          -> TMEM columns 0..127
 //   softmax        row max / exp2 / row sum in registers (log2 domain, online rescale);
-//                  P goes back into tensor memory as packed 16-bit pairs, over the first 32
-//                  columns of the S buffer it was computed from (tcgen05.st: a thread writes
-//                  its own lane, no shared-memory traffic)
-//   O += P V       4 MMAs (M128 N128 K16) with P as the A operand from tensor memory and the
+//                  P goes back into tensor memory as packed 16-bit pairs, a thread's over the first
+//                  half of its own S (tcgen05.st: a thread writes its own lane, no shared-memory traffic)
+//   O += P V       8 MMAs (M128 N128 K16) with P as the A operand from tensor memory and the
 //                  value tile as an MN-major B operand from shared memory, accumulating over
 //                  all tiles                                                   -> TMEM columns 128..255
+//
+// What bounds it: a CTA's chain is serial (S, softmax, product), since S, P and O fill its half of tensor memory, and
+// only the other CTA on the SM works meanwhile.  A tile needs the tensor core and the special-function unit for
+// 1024 cycles each, and takes 1840 (both are busy a little over half of the time).  128-key tiles, because every MMA
+// of S reads its 4 KB slice of Q again: with 64 keys it moved 6 KB of shared memory for 32 cycles of
+// arithmetic.  K and V need one stage each: a key tile is refilled during the softmax, a value tile during the
+// next S and softmax.  Two threads per row, because one needs 168 registers for its 128 logits and leaves the
+// compiler no room to interleave (2.4 cycles of fixed latency per instruction); two need 96.
+// us for 2999 / 8192 / 16384 tokens x 32 heads: 64-key tiles, four softmax warps 129 / 591 / 2068; 128-key tiles
+// 104 / 512 / 1936; with eight softmax warps 100 / 492 / 1866 (1180 TFLOP/s).
 //
 // O never leaves tensor memory until the end: the exponentials of a row are taken against a
 // reference that follows the row maximum lazily, and O is rescaled in place (tcgen05.ld / st)
 // only when a tile's maximum outgrows the reference by more than 2^8 - after the first tiles,
-// hardly ever.  The loop is software-pipelined so that the tensor core is not waited on in
-// line: S of tile j+1 is issued (into the second S buffer) before the softmax of tile j starts,
-// and the product of tile j runs during the softmax of tile j+1.  The tensor core executes in
-// issue order, so S of tile j+2, which overwrites the buffer P of tile j lies in, runs after
-// the product that reads it.  Key and value tiles are double-buffered (a key stage is refilled
-// as soon as its S is complete, a value stage once its product is).  Every wait on an
-// mbarrier is bounded: a wait that runs out sets DA_STATUS_WAIT_TIMEOUT and a flag that makes
-// both roles leave their loops; the CTA then frees its tensor memory and returns.
+// hardly ever.  Every wait on an mbarrier is bounded: a wait that runs out sets
+// DA_STATUS_WAIT_TIMEOUT and a flag that makes all roles leave their loops; the CTA then frees its tensor
+// memory and returns.
 //
 // GQA: query head hq reads KV head hq / rep.  Causal: key tiles above the diagonal are
 // skipped, the diagonal tile is masked per element.  Rows past the end of the prompt are
@@ -44,24 +40,29 @@
 
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "da_common.cuh"
 
 namespace da {
 
-constexpr int kPfRows = 128;    // query rows per CTA (= softmax threads, = TMEM lanes)
-constexpr int kPfThreads = kPfRows + 64;   // plus the warp that issues the MMAs and the warp that issues the copies
-constexpr int kPfKeys = 64;     // keys per tile
+constexpr int kPfRows = 128;    // query rows per CTA (= TMEM lanes)
+constexpr int kPfSoftmaxWarps = 8;         // two per 32 rows: each takes half of a tile's keys
+constexpr int kPfThreads = kPfSoftmaxWarps * 32 + 64;   // plus the warp that issues the MMAs and the warp that issues the copies
+constexpr int kPfKeys = 128;    // keys per tile
 constexpr int kPfDim = 128;     // head_dim
 constexpr int kPfQBoxBytes = kPfRows * 128;           // one TMA box of Q: 128 rows x 64 elements
 constexpr int kPfQTileBytes = 2 * kPfQBoxBytes;       // 128 x 128 elements
-constexpr int kPfBoxBytes = kPfKeys * 128;            // one TMA box of K or V: 64 rows x 64 elements
-constexpr int kPfTileBytes = 2 * kPfBoxBytes;         // 64 x 128 elements
-constexpr int kPfSmemBytes = kPfQTileBytes + 4 * kPfTileBytes + 1024;   // Q, K x2, V x2, alignment slack
-constexpr uint32_t kPfTmemCols = 256;            // two S buffers of 64 columns (P over them), the product
+constexpr int kPfBoxBytes = kPfKeys * 128;            // one TMA box of K or V: 128 rows x 64 elements
+constexpr int kPfTileBytes = 2 * kPfBoxBytes;         // 128 x 128 elements
+constexpr int kPfSmemBytes = kPfQTileBytes + 2 * kPfTileBytes + 1024;   // Q, K, V, alignment slack
+constexpr long long kPfL2Share = 32ll << 20;    // of the keys and values that a launch works on at a time
+constexpr uint32_t kPfTmemCols = 256;            // S (P over its first half), the product
 
 struct PrefillParams {
     void *out;              // (S, Hq, D)
     int seq_len, n_q_heads, rep;
+    int n_qtiles, heads_per_group;
     float scale_log2;
     int32_t *status;
 };
@@ -168,38 +169,33 @@ __device__ __forceinline__ void tmem_wait32(uint32_t (&r)[32]) {
         : "memory");
 }
 
-__device__ __forceinline__ void tmem_store32(uint32_t taddr, const uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_store16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
-          "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
-          "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
 }
 
-__device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// f(chunk, values) for the four 32-column chunks starting at taddr, the load of a chunk in
-// flight while the previous one is processed
-template <typename F>
-__device__ __forceinline__ void tmem_for_chunks(uint32_t taddr, F f) {
-    uint32_t ra[32], rb[32];
-    tmem_issue32(taddr, ra);
-    tmem_wait32(ra);
-    tmem_issue32(taddr + 32, rb);
-    f(0, ra);
-    tmem_wait32(rb);
-    tmem_issue32(taddr + 64, ra);
-    f(1, rb);
-    tmem_wait32(ra);
-    tmem_issue32(taddr + 96, rb);
-    f(2, ra);
-    tmem_wait32(rb);
-    f(3, rb);
+// Eight columns there and back (the rescaling of O, while a row of S fills the registers).
+__device__ __forceinline__ void tmem_scale8(uint32_t taddr, float f) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+                 :
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * f);
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
 }
+
+__device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Shared-memory matrix descriptors, 128-byte swizzle, version 1 (Blackwell).  Addresses and
 // offsets in units of 16 bytes.
@@ -265,30 +261,35 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                             ~(uintptr_t)1023);
     unsigned char *sQ = smem;
-    unsigned char *sK = sQ + kPfQTileBytes;           // two stages
-    unsigned char *sV = sK + 2 * kPfTileBytes;        // two stages
-    __shared__ __align__(8) uint64_t bar_q, bar_k[2], bar_v[2], bar_s[2], bar_p[2], bar_pv;
+    unsigned char *sK = sQ + kPfQTileBytes;
+    unsigned char *sV = sK + kPfTileBytes;
+    __shared__ __align__(8) uint64_t bar_q, bar_k, bar_v, bar_s, bar_p, bar_pv, bar_x[kPfRows / 32];
+    __shared__ float sh_x[2][2][kPfRows];     // what the two threads of a row tell each other: [tile parity][half][row]
     __shared__ uint32_t tmem_holder;
     __shared__ int sh_abort;
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
-    const int n_qtiles = gridDim.x;
-    const int qt = n_qtiles - 1 - blockIdx.x;     // the tiles with the most keys start first
-    const int hq = blockIdx.y;
+    // Within a group of heads the tiles with the most keys start first, so that what is left for the end of
+    // the launch are the short ones.
+    int qt, hq;
+    {
+        const int per_group = p.n_qtiles * p.heads_per_group;
+        const int group = blockIdx.x / per_group, at = blockIdx.x % per_group;
+        qt = p.n_qtiles - 1 - at / p.heads_per_group;
+        hq = group * p.heads_per_group + at % p.heads_per_group;
+    }
     const int hk = hq / p.rep;
     const int q0 = qt * kPfRows;
     constexpr bool bf16 = BF16;
 
     if (tid == 0) {
         mbar_init(&bar_q, 1);
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(&bar_k[b], 1);
-            mbar_init(&bar_v[b], 1);
-            mbar_init(&bar_s[b], 1);
-            mbar_init(&bar_p[b], kPfRows);     // every softmax thread arrives
-        }
+        mbar_init(&bar_k, 1);
+        mbar_init(&bar_v, 1);
+        mbar_init(&bar_s, 1);
+        mbar_init(&bar_p, kPfSoftmaxWarps);     // every softmax warp arrives
+        for (int i = 0; i < kPfRows / 32; ++i) mbar_init(&bar_x[i], 2);
         mbar_init(&bar_pv, 1);
         mbar_fence_init();
         sh_abort = 0;
@@ -299,12 +300,11 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_holder;
-    // columns: S of even tiles 0..63, S of odd tiles 64..127 (P over the first 32 of each), O 128..255
-    const uint32_t tmem_o = 2 * kPfKeys;
+    // columns: S 0..127 (P over the first half of either half: 0..31, 64..95), O 128..255
+    const uint32_t tmem_o = kPfKeys;
 
-    // keys 0 .. q0 + 127 are visible to this tile's rows
-    const int last_key = min(p.seq_len, q0 + kPfRows);
-    const int n_tiles = (last_key + kPfKeys - 1) / kPfKeys;
+    // keys 0 .. q0 + 127 are visible to this tile's rows: the last key tile is the diagonal one
+    const int n_tiles = qt + 1;
     volatile int *abort_flag = &sh_abort;
     // a wait that ran out: say so, and let every role leave its loop at its next tile
     auto give_up = [&]() {
@@ -312,10 +312,9 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         *abort_flag = 1;
     };
 
-    if (warp == kPfRows / 32 + 1) {
+    if (warp == kPfSoftmaxWarps + 1) {
         // =================== the copy warp: every TMA copy, by one lane ===================================
-        // Key tile j+2 goes into the stage of tile j once S(j) is complete, value tile j+2 into the stage
-        // of tile j once the product of tile j is.
+        // Key tile j+1 goes where tile j was once S(j) is complete, value tile j+1 once the product of tile j is.
         if ((tid & 31) == 0) {
             auto load_tile = [&](unsigned char *dst, const CUtensorMap *map, int j, uint64_t *bar) {
                 mbar_arrive_expect_tx(bar, kPfTileBytes);
@@ -325,80 +324,74 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             mbar_arrive_expect_tx(&bar_q, kPfQTileBytes);
             tma_load_3d(sQ, &map_q, 0, hq, q0, &bar_q);
             tma_load_3d(sQ + kPfQBoxBytes, &map_q, 64, hq, q0, &bar_q);
-            load_tile(sK, &map_k, 0, &bar_k[0]);
-            load_tile(sV, &map_v, 0, &bar_v[0]);
-            if (n_tiles > 1) {
-                load_tile(sK + kPfTileBytes, &map_k, 1, &bar_k[1]);
-                load_tile(sV + kPfTileBytes, &map_v, 1, &bar_v[1]);
-            }
+            load_tile(sK, &map_k, 0, &bar_k);
+            load_tile(sV, &map_v, 0, &bar_v);
             bool ok = true;
-            for (int j = 0; ok && j + 2 < n_tiles; ++j) {
-                const int b = j & 1;
+            for (int j = 0; ok && j + 1 < n_tiles; ++j) {
                 if (*abort_flag) break;
-                ok = mbar_wait_bounded(&bar_s[b], (uint32_t)((j >> 1) & 1));
+                ok = mbar_wait_bounded(&bar_s, (uint32_t)(j & 1));
                 if (!ok) break;
-                load_tile(sK + b * kPfTileBytes, &map_k, j + 2, &bar_k[b]);
+                load_tile(sK, &map_k, j + 1, &bar_k);
                 ok = mbar_wait_bounded(&bar_pv, (uint32_t)(j & 1));
                 if (!ok) break;
-                load_tile(sV + b * kPfTileBytes, &map_v, j + 2, &bar_v[b]);
+                load_tile(sV, &map_v, j + 1, &bar_v);
             }
             if (!ok) give_up();
         }
-    } else if (warp == kPfRows / 32) {
+    } else if (warp == kPfSoftmaxWarps) {
         // =================== the issuing warp: every MMA, by one lane =====================================
-        // Its instruction stream is the pace of the whole CTA, so everything that can be is computed
-        // before the loop: the operand descriptors of both stages (an MMA's own is a 64-bit add away).
+        // Everything that can be is computed before the loop: the operand descriptors (an MMA's own is a
+        // 64-bit add away).
         if ((tid & 31) == 0) {
             const uint32_t idesc_s = instr_desc(bf16, false, kPfKeys), idesc_o = instr_desc(bf16, true, kPfDim);
-            const uint64_t dq = desc_k_major(smem_addr(sQ));
-            const uint64_t dk0 = desc_k_major(smem_addr(sK)), dk1 = desc_k_major(smem_addr(sK + kPfTileBytes));
-            const uint64_t dv0 = desc_mn_major(smem_addr(sV)), dv1 = desc_mn_major(smem_addr(sV + kPfTileBytes));
-            // S(j) = Q K(j)^T into the S buffer of j's parity; K(j) has arrived when this is called.  That
-            // buffer's last readers were the softmax of tile j-2 (done: its P was waited for before the
-            // product of tile j-2 was issued) and that product (issued earlier: the tensor core runs in order).
-            auto issue_s = [&](int j) {
+            const uint64_t dq = desc_k_major(smem_addr(sQ)), dk = desc_k_major(smem_addr(sK));
+            const uint64_t dv = desc_mn_major(smem_addr(sV));
+            // S(j) = Q K(j)^T; K(j) has arrived when this is called.  The columns it overwrites were last read by the
+            // softmax of tile j-1 (done: its P was waited for before the product of tile j-1 was issued) and by that
+            // product (issued earlier: the tensor core runs in order).
+            auto issue_s = [&]() {
                 tc_fence_after();
-                const uint64_t kb = (j & 1) ? dk1 : dk0;
-                const uint32_t d = tmem + (j & 1) * kPfKeys;
 #pragma unroll
                 for (int ks = 0; ks < kPfDim / 16; ++ks) {
                     const uint32_t a_off = ((ks >> 2) * kPfQBoxBytes + (ks & 3) * 32) >> 4;
                     const uint32_t b_off = ((ks >> 2) * kPfBoxBytes + (ks & 3) * 32) >> 4;
-                    if (ks == 0) tc_mma_c<false>(d, dq + a_off, kb + b_off, idesc_s);
-                    else tc_mma_c<true>(d, dq + a_off, kb + b_off, idesc_s);
+                    if (ks == 0) tc_mma_c<false>(tmem, dq + a_off, dk + b_off, idesc_s);
+                    else tc_mma_c<true>(tmem, dq + a_off, dk + b_off, idesc_s);
                 }
-                tc_commit(&bar_s[j & 1]);
+                tc_commit(&bar_s);
             };
-            bool ok = mbar_wait_bounded(&bar_q, 0) && mbar_wait_bounded(&bar_k[0], 0);
-            if (ok) issue_s(0);
+            bool ok = mbar_wait_bounded(&bar_q, 0) && mbar_wait_bounded(&bar_k, 0);
+            if (ok) issue_s();
             for (int j = 0; ok && j < n_tiles; ++j) {
-                const int b = j & 1;
-                const uint32_t use = (uint32_t)((j >> 1) & 1);     // parity of this use of a two-deep buffer
+                const uint32_t use = (uint32_t)(j & 1);
                 if (*abort_flag) break;
-                if (j + 1 < n_tiles) {
-                    ok = mbar_wait_bounded(&bar_k[b ^ 1], (uint32_t)(((j + 1) >> 1) & 1));
-                    if (!ok) break;
-                    issue_s(j + 1);
-                }
-                // O += P(j) V(j) once every softmax thread has written its row of P (and has
-                // rescaled its row of O if it had to)
-                ok = mbar_wait_bounded(&bar_p[b], use) && mbar_wait_bounded(&bar_v[b], use);
+                // O += P(j) V(j) once every softmax warp has written its part of P (and has rescaled its part of O
+                // if it had to)
+                ok = mbar_wait_bounded(&bar_v, use) && mbar_wait_bounded(&bar_p, use);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t a0 = tmem + (uint32_t)b * kPfKeys;
-                const uint64_t vb = b ? dv1 : dv0;
-                if (j == 0) tc_mma_a_tmem_c<false>(tmem + tmem_o, a0, vb, idesc_o);
-                else tc_mma_a_tmem_c<true>(tmem + tmem_o, a0, vb, idesc_o);
+                if (j == 0) tc_mma_a_tmem_c<false>(tmem + tmem_o, tmem, dv, idesc_o);
+                else tc_mma_a_tmem_c<true>(tmem + tmem_o, tmem, dv, idesc_o);
 #pragma unroll
                 for (int ks = 1; ks < kPfKeys / 16; ++ks)      // 16 keys further down the tile per step
-                    tc_mma_a_tmem_c<true>(tmem + tmem_o, a0 + ks * 8, vb + ((ks * 16 * 128) >> 4), idesc_o);
+                    tc_mma_a_tmem_c<true>(tmem + tmem_o, tmem + (ks >> 2) * (kPfKeys / 2) + (ks & 3) * 8,
+                                          dv + ((ks * 16 * 128) >> 4), idesc_o);
                 tc_commit(&bar_pv);
+                if (j + 1 < n_tiles) {
+                    ok = mbar_wait_bounded(&bar_k, use ^ 1u);
+                    if (!ok) break;
+                    issue_s();
+                }
             }
             if (!ok) give_up();
         }
     } else {
-        // =================== the softmax warps: thread t = query row t = TMEM lane t ===================
-        const uint32_t tmem_row = tmem + ((uint32_t)(warp * 32) << 16);   // this warp's 32 lanes
+        // ====== the softmax warps: two threads per query row (= TMEM lane), one per half of a tile's keys ======
+        const int group = warp & 3, half = warp >> 2;     // 32 rows, which a warp reaches by its number modulo 4
+        const int lane = tid & 31;
+        const int row = group * 32 + lane;
+        const uint32_t tmem_row = tmem + ((uint32_t)(group * 32) << 16);   // this warp's 32 lanes
+        const uint32_t tmem_s = tmem_row + half * (kPfKeys / 2);
         // m_used: the (log2-domain) reference the exponentials of this row are taken against.  It
         // follows the row maximum lazily: O, which accumulates in tensor memory over all tiles, is
         // rescaled only when a tile's maximum exceeds the reference by more than 8 (probabilities
@@ -409,75 +402,66 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         constexpr float kRescaleSlack = 8.f;
         bool ok = true;
 
-        for (int j = 0; j < n_tiles; ++j) {
-            const int b = j & 1;
-            const uint32_t use = (uint32_t)((j >> 1) & 1);
-            if (*abort_flag) {
-                ok = false;
-                break;
-            }
-            // S(j) was committed after the product of tile j-2 was issued: P's buffer b is free too
-            ok = mbar_wait_bounded(&bar_s[b], use);
-            if (!__all_sync(DA_FULL_MASK, ok)) {
-                ok = false;
-                break;
-            }
+        // v to the row's other thread, and its v back; `use` counts the exchanges
+        auto exchange = [&](float v, int use, float &other) -> bool {
+            sh_x[use & 1][half][row] = v;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar_x[group]);
+            const bool there = mbar_wait_bounded(&bar_x[group], (uint32_t)(use & 1));
+            other = sh_x[use & 1][half ^ 1][row];
+            return __all_sync(DA_FULL_MASK, there);
+        };
+
+        // One key tile; DIAG: the last one, of which row t sees the keys 0 .. t.  Chunks of 32 keys: of the diagonal
+        // tile a warp sees the chunks before its rows' own whole, their own up to the diagonal, and none after it.
+        auto tile = [&](int j, auto diag) -> bool {
+            constexpr bool DIAG = decltype(diag)::value;
+            // S(j) complete also says that the product of tile j-1 is: O may be rescaled
+            bool ready = mbar_wait_bounded(&bar_s, (uint32_t)(j & 1));
+            // The wait on the last product, after the loop, must not return on the phase two before it: the phase
+            // between them is waited for here, where this thread's own P, still to come, keeps the last one from
+            // completing (waited for later, it might be past already, and a parity names only every other phase).
+            if (DIAG && j > 0) ready = ready && mbar_wait_bounded(&bar_pv, (uint32_t)((j - 1) & 1));
+            if (!__all_sync(DA_FULL_MASK, ready)) return false;
             tc_fence_after();
 
-            // ---- this thread's row of S, read once ------------------------------------------------
-            const uint32_t tmem_s = (uint32_t)b * kPfKeys;
-            const int qpos = q0 + tid;
-            const int key0 = j * kPfKeys;
-            const bool diagonal = key0 + kPfKeys - 1 > q0;      // some key of the tile is masked for some row
-            const int n_vis = diagonal ? min(max(qpos - key0 + 1, 0), kPfKeys) : kPfKeys;   // keys this row sees
-            uint32_t s0[32], s1[32];
-            tmem_issue32(tmem_row + tmem_s, s0);
-            tmem_issue32(tmem_row + tmem_s + 32, s1);
-            tmem_wait32(s0);
-            tmem_wait32(s1);
-            float mx = -INFINITY;
-            auto chunk_max = [&](int c, const uint32_t (&s)[32]) {
-                if (!diagonal) {
-                    float m1 = -INFINITY;    // two chains of three-input maxima
+            // ---- this thread's half of the row of S, read once ----------------------------------------
+            uint32_t s[2][32];
+            float mx = -INFINITY, mx1 = -INFINITY;    // two chains of three-input maxima
+            tmem_issue32(tmem_s, s[0]);
+            tmem_issue32(tmem_s + 32, s[1]);
+            tmem_wait32(s[0]);
+            tmem_wait32(s[1]);
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4) {
-                        mx = max3(mx, __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
-                        m1 = max3(m1, __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
-                    }
-                    mx = fmaxf(mx, m1);
-                } else {
+            for (int cc = 0; cc < 2; ++cc) {
+                const int c = 2 * half + cc;
+                if (DIAG && c > group) continue;
+                if (DIAG && c == group) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i)
-                        if (c * 32 + i < n_vis) mx = fmaxf(mx, __uint_as_float(s[i]));
+                        if (i <= lane) mx = fmaxf(mx, __uint_as_float(s[cc][i]));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4) {
+                        mx = max3(mx, __uint_as_float(s[cc][i]), __uint_as_float(s[cc][i + 1]));
+                        mx1 = max3(mx1, __uint_as_float(s[cc][i + 2]), __uint_as_float(s[cc][i + 3]));
+                    }
                 }
-            };
-            chunk_max(0, s0);
-            chunk_max(1, s1);
-            const float m_tile = mx * p.scale_log2;
+            }
+            float m_half = fmaxf(mx, mx1) * p.scale_log2, m_other;
+            if (!exchange(m_half, j, m_other)) return false;
+            const float m_tile = fmaxf(m_half, m_other);
 
             // ---- move the reference if this tile outgrows it (whole warp together: the tensor-memory
-            //      accesses are warp-wide) ---------------------------------------------------------------
+            //      accesses are warp-wide; the two warps of the rows come to the same result) -----------------
             const bool grow = m_tile > m_used + kRescaleSlack;     // also true on the first tile (-inf)
             if (__any_sync(DA_FULL_MASK, grow)) {
                 const float m_next = grow ? m_tile : m_used;
                 const float alpha = (m_used == -INFINITY) ? 0.f : fast_exp2(m_used - m_next);
                 if (j > 0) {
-                    // O holds the products up to tile j-1: wait for the last of them, scale the row
-                    ok = mbar_wait_bounded(&bar_pv, (uint32_t)((j - 1) & 1));
-                    if (!__all_sync(DA_FULL_MASK, ok)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-#pragma unroll
-                    for (int c = 0; c < kPfDim / 32; ++c) {
-                        uint32_t t[32];
-                        tmem_issue32(tmem_row + tmem_o + c * 32, t);
-                        tmem_wait32(t);
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) t[i] = __float_as_uint(__uint_as_float(t[i]) * alpha);
-                        tmem_store32(tmem_row + tmem_o + c * 32, t);
-                    }
+#pragma unroll 1
+                    for (int c = 0; c < kPfDim / 2; c += 8)
+                        tmem_scale8(tmem_row + tmem_o + half * (kPfDim / 2) + c, alpha);
                     tmem_wait_store();
                 }
                 l_run *= alpha;
@@ -486,57 +470,70 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             const float m_ref = (m_used == -INFINITY) ? 0.f : m_used;
 
             // ---- P = exp2(S * scale - reference) as packed 16-bit pairs into tensor memory, over this
-            //      row's own (already read) S --------------------------------------------------------------
-            uint32_t packed[32];
+            //      thread's own (already read) S ----------------------------------------------------------------
             unsigned long long sum2 = f32x2(0.f, 0.f);     // the row sum, even and odd keys apart
             const unsigned long long scale2 = f32x2(p.scale_log2, p.scale_log2), mref2 = f32x2(-m_ref, -m_ref);
-            auto chunk_p = [&](int c, const uint32_t (&s)[32]) {
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    float x0, x1;
-                    f32x2_split(fma2(f32x2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), scale2, mref2), x0, x1);
-                    float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-                    if (diagonal) {
-                        if (c * 32 + i >= n_vis) p0 = 0.f;
-                        if (c * 32 + i + 1 >= n_vis) p1 = 0.f;
+            for (int cc = 0; cc < 2; ++cc) {
+                const int c = 2 * half + cc;
+                uint32_t packed[16];
+                if (DIAG && c > group) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) packed[i] = 0u;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        float x0, x1;
+                        f32x2_split(fma2(f32x2(__uint_as_float(s[cc][i]), __uint_as_float(s[cc][i + 1])), scale2, mref2), x0, x1);
+                        float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
+                        if (DIAG && c == group) {
+                            if (i > lane) p0 = 0.f;
+                            if (i + 1 > lane) p1 = 0.f;
+                        }
+                        sum2 = add2(sum2, f32x2(p0, p1));
+                        packed[i >> 1] = pack16<BF16>(p0, p1);
                     }
-                    sum2 = add2(sum2, f32x2(p0, p1));
-                    packed[c * 16 + (i >> 1)] = pack16<BF16>(p0, p1);
                 }
-            };
-            chunk_p(0, s0);
-            chunk_p(1, s1);
-            tmem_store32(tmem_row + tmem_s, packed);
+                tmem_store16(tmem_s + cc * 16, packed);
+            }
             tmem_wait_store();
+            tc_fence_before();            // this thread's tensor-memory accesses are ordered before the arrival
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar_p);
             {
                 float s_even, s_odd;
                 f32x2_split(sum2, s_even, s_odd);
                 l_run += s_even + s_odd;
             }
-            tc_fence_before();            // this thread's tensor-memory accesses are ordered before the arrival
-            mbar_arrive(&bar_p[b]);
-        }
+            return true;
+        };
+        for (int j = 0; ok && j + 1 < n_tiles; ++j) ok = *abort_flag == 0 && tile(j, std::false_type());
+        ok = ok && *abort_flag == 0;
+        ok = __all_sync(DA_FULL_MASK, ok) && tile(n_tiles - 1, std::true_type());
 
-        // ---- this row of O, normalised ---------------------------------------------------------------
-        // A warp may get here one tile ahead of the slowest one, before the product of tile n-2 has even been
-        // issued; S(n-1) only vouches for the product of tile n-3, whose phase has the parity of the last one's.
-        // So both outstanding phases are waited for in turn: a wait on the last parity alone returns at once on
-        // the phase before the previous one, and the row would leave without its two last (diagonal) tiles.
-        if (ok && n_tiles > 0) {
-            if (n_tiles > 1) ok = mbar_wait_bounded(&bar_pv, (uint32_t)((n_tiles - 2) & 1));
-            ok = ok && mbar_wait_bounded(&bar_pv, (uint32_t)((n_tiles - 1) & 1));
+        // ---- this thread's half of the row of O, normalised --------------------------------------------
+        float l_other = 0.f;
+        ok = ok && exchange(l_run, n_tiles, l_other);
+        // (the phase before this one was waited for in the last tile)
+        if (ok) {
+            ok = mbar_wait_bounded(&bar_pv, (uint32_t)((n_tiles - 1) & 1));
             ok = __all_sync(DA_FULL_MASK, ok);
         }
         if (!ok) {
-            if ((tid & 31) == 0) give_up();
+            if (lane == 0) give_up();
         } else {
             tc_fence_after();
-            const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-            const bool live = q0 + tid < p.seq_len;
+            const float l = half == 0 ? l_run + l_other : l_other + l_run;
+            const float inv = l > 0.f ? 1.f / l : 0.f;
+            const bool live = q0 + row < p.seq_len;
             unsigned char *dst = static_cast<unsigned char *>(p.out) +
-                                 ((size_t)(live ? q0 + tid : 0) * p.n_q_heads + hq) * kPfDim * 2;
-            tmem_for_chunks(tmem_row + tmem_o, [&](int c, const uint32_t (&t)[32]) {
-                if (!live) return;
+                                 ((size_t)(live ? q0 + row : 0) * p.n_q_heads + hq) * kPfDim * 2 + half * kPfDim;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                uint32_t t[32];
+                tmem_issue32(tmem_row + tmem_o + half * (kPfDim / 2) + c * 32, t);
+                tmem_wait32(t);
+                if (!live) continue;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const int i = 8 * q;
@@ -546,7 +543,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                                    pack16<BF16>(__uint_as_float(t[i + 4]) * inv, __uint_as_float(t[i + 5]) * inv),
                                    pack16<BF16>(__uint_as_float(t[i + 6]) * inv, __uint_as_float(t[i + 7]) * inv));
                 }
-            });
+            }
         }
     }
     tc_fence_before();
@@ -630,7 +627,16 @@ extern "C" int da_prefill_attention(const void *q, const void *k, const void *v,
     p.rep = n_q_heads / n_kv_heads;
     p.scale_log2 = 1.4426950408889634f / sqrtf((float)head_dim);
     p.status = status;
-    const dim3 grid((seq_len + da::kPfRows - 1) / da::kPfRows, n_q_heads);
+    p.n_qtiles = (seq_len + da::kPfRows - 1) / da::kPfRows;
+    // As many KV heads at a time as keep their keys and values in a quarter of the L2 cache (all heads of a short
+    // prompt: the launch then ends with its shortest tiles); a divisor of the head count.
+    const long long kv_bytes = 2ll * seq_len * head_dim * 2;
+    int kv_heads = n_kv_heads;
+    while (kv_heads > 1 && (n_kv_heads % kv_heads != 0 || kv_heads * kv_bytes > da::kPfL2Share)) --kv_heads;
+    p.heads_per_group = kv_heads * p.rep;
+    const long long ctas = (long long)p.n_qtiles * n_q_heads;
+    if (ctas > 0x7fffffffll) return DA_ERR_UNSUPPORTED;
+    const dim3 grid((unsigned)ctas);
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     if (bf16) da::prefill_attention_kernel<true><<<grid, da::kPfThreads, da::kPfSmemBytes, cs>>>(mq, mk, mv, p);
     else da::prefill_attention_kernel<false><<<grid, da::kPfThreads, da::kPfSmemBytes, cs>>>(mq, mk, mv, p);

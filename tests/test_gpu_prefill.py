@@ -124,3 +124,25 @@ def test_operator_prefill_then_generate(da):
     step2 = lib_call(q1, k1, v1, start_pos=s, stage="generate")
     assert torch.equal(step, step2)      # both built the same cache from the same keys and values
     m.check_status()
+
+
+def test_prefill_kernel_heads_in_groups(da):
+    """A prompt whose keys and values outgrow the share of L2 a launch works on is taken a few KV heads at a time
+    (here 6 heads of 8.4 MB in two groups of 3): every (head, row tile) is covered once, edges of tiles included."""
+    from dram_attention_b200 import _native
+    s, hq, hk = 16384 + 5, 12, 6
+    g = torch.Generator(device=DEV).manual_seed(4)
+    q, k, v = (torch.randn(s, h, 128, generator=g, device=DEV).to(torch.bfloat16) for h in (hq, hk, hk))
+    out = torch.full_like(q, float("nan"))
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    _native.check(_native.lib().da_prefill_attention(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), s, hq, hk, 128, hq * 128, hk * 128,
+        _native.dtype_code(q.dtype), status.data_ptr(), _native.stream_ptr()))
+    torch.cuda.synchronize()
+    assert int(status) == 0 and bool(torch.isfinite(out.float()).all())
+    rows = torch.tensor([0, 1, 31, 32, 127, 128, 129, 255, 256, 8191, 8192, 16255, 16256, 16383, 16384, s - 1])
+    seen = torch.arange(s, device=DEV)[None] <= rows.to(DEV)[:, None]
+    for h in range(hq):
+        sc = q[rows, h].double() @ k[:, h // 2].double().T / 128 ** 0.5
+        ref = torch.softmax(sc.masked_fill(~seen, float("-inf")), -1) @ v[:, h // 2].double()
+        _close(out[rows, h], ref, q.dtype)
