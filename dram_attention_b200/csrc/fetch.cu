@@ -99,10 +99,121 @@ __global__ void build_pages_kernel(const T *__restrict__ k, const T *__restrict_
     }
 }
 
+// The same pass with 16 bytes per thread and load: 2 * chunks consecutive threads take one page of one head
+// (chunks = 16-byte pieces of a row), thread c the c-th piece of its key row, then value row, of every token, so that
+// a token leaves as one contiguous run of both rows and a thread sees all the keys of its channels (no exchange for
+// the summaries).  For rows of whole 16-byte pieces, at most 1 KB long, on 16-byte boundaries.  Neighbouring groups take the heads of a page, whose rows are neighbours in the prompt's keys.
+constexpr int kBuildThreads = 128;
+constexpr int kBuildUnroll = 4;
+constexpr int kBuildSms = 148;
+// With pages in host memory the link is the bound, and a few CTAs keep it busy: 117 MB in 2269, 2254, 2255 us with
+// 8, 24, 148 CTAs (52 GB/s; two bytes per thread and a CTA per page: 2678).  24 of them leave the prefill attention
+// its SMs when the two run side by side.
+constexpr int kBuildLinkCtas = 24;
+
+// Per element of a 32-bit word: the smaller (larger) one as it lies in memory, the one that was there first when they
+// do not compare (zeros of either sign, NaN).
+template <typename T> __device__ __forceinline__ void keep_extremes(uint32_t w, uint32_t &mn, uint32_t &mx) {
+    if constexpr (sizeof(T) == 4) {
+        const float f = __uint_as_float(w);
+        if (f < __uint_as_float(mn)) mn = w;
+        if (f > __uint_as_float(mx)) mx = w;
+    } else {
+        float f0, f1, a0, a1, b0, b1;
+        unpack2<T>(w, f0, f1);
+        unpack2<T>(mn, a0, a1);
+        unpack2<T>(mx, b0, b1);
+        mn = (f0 < a0 ? w & 0xffffu : mn & 0xffffu) | (f1 < a1 ? w & 0xffff0000u : mn & 0xffff0000u);
+        mx = (f0 > b0 ? w & 0xffffu : mx & 0xffffu) | (f1 > b1 ? w & 0xffff0000u : mx & 0xffff0000u);
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kBuildThreads)
+build_pages_vec_kernel(const unsigned char *__restrict__ k, const unsigned char *__restrict__ v, long long tok_stride,
+                       long long head_stride, uint4 *__restrict__ dram, uint4 *__restrict__ summaries,
+                       uint4 *__restrict__ slots, int n_kv_heads, int n_pages, int n_slots, int page_size, int chunks) {
+    const int lanes = 2 * chunks;
+    const int groups = kBuildThreads / lanes;
+    const int g = threadIdx.x / lanes;
+    if (g >= groups) return;
+    const int c = threadIdx.x - g * lanes;
+    const bool is_key = c < chunks;
+    if (!is_key && !dram && !slots) return;   // summaries alone
+    const unsigned char *rows = (is_key ? k : v) + (size_t)(is_key ? c : c - chunks) * 16;
+    const int first_resident = n_pages - n_slots;
+    const long long page_vecs = (long long)page_size * lanes;
+    const unsigned items = (unsigned)n_pages * (unsigned)n_kv_heads;
+    for (unsigned item = blockIdx.x * groups + g; item < items; item += gridDim.x * groups) {
+        const int page = (int)(item / (unsigned)n_kv_heads);
+        const int h = (int)(item % (unsigned)n_kv_heads);
+        const unsigned char *src = rows + (long long)page * page_size * tok_stride + (long long)h * head_stride;
+        uint4 *pg = dram ? dram + ((long long)h * n_pages + page) * page_vecs + c : nullptr;
+        uint4 *sl = slots && page >= first_resident
+                        ? slots + ((long long)h * n_slots + (page - first_resident)) * page_vecs + c : nullptr;
+        uint32_t mn[4] = {0, 0, 0, 0}, mx[4] = {0, 0, 0, 0};
+#pragma unroll 1
+        for (int t0 = 0; t0 < page_size; t0 += kBuildUnroll) {
+            const int n = page_size - t0;
+            uint4 r[kBuildUnroll];
+#pragma unroll
+            for (int u = 0; u < kBuildUnroll; ++u) {
+                if (u < n) r[u] = *reinterpret_cast<const uint4 *>(src);
+                src += tok_stride;
+            }
+            if (pg) {
+#pragma unroll
+                for (int u = 0; u < kBuildUnroll; ++u) {
+                    if (u < n) *pg = r[u];
+                    pg += lanes;
+                }
+            }
+            if (sl) {
+#pragma unroll
+                for (int u = 0; u < kBuildUnroll; ++u) {
+                    if (u < n) *sl = r[u];
+                    sl += lanes;
+                }
+            }
+            if (!summaries || !is_key) continue;
+#pragma unroll
+            for (int u = 0; u < kBuildUnroll; ++u) {
+                if (u >= n) break;
+                const uint32_t w[4] = {r[u].x, r[u].y, r[u].z, r[u].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (u == 0 && t0 == 0) mn[i] = mx[i] = w[i];
+                    keep_extremes<T>(w[i], mn[i], mx[i]);
+                }
+            }
+        }
+        if (summaries && is_key) {
+            uint4 *sm = summaries + ((long long)h * n_pages + page) * lanes + c;
+            sm[0] = make_uint4(mn[0], mn[1], mn[2], mn[3]);
+            sm[chunks] = make_uint4(mx[0], mx[1], mx[2], mx[3]);
+        }
+    }
+}
+
 template <typename T>
 static cudaError_t launch_build(const void *k, const void *v, long long tok_stride, long long head_stride,
                                 void *dram, void *summaries, void *slots, int n_kv_heads, int n_pages,
                                 int n_slots, int page_size, int head_dim, cudaStream_t stream) {
+    constexpr long long E = (long long)sizeof(T);
+    const int chunks = (int)(head_dim * E / 16);
+    const uintptr_t all = (uintptr_t)k | (uintptr_t)v | (uintptr_t)dram | (uintptr_t)summaries | (uintptr_t)slots |
+                          (uintptr_t)(tok_stride * E) | (uintptr_t)(head_stride * E) | (uintptr_t)(head_dim * E);
+    if ((all & 15) == 0 && 2 * chunks <= kBuildThreads && (long long)n_pages * n_kv_heads <= 0x7fffffffll) {
+        const long long groups = kBuildThreads / (2 * chunks);
+        long long ctas = ((long long)n_pages * n_kv_heads + groups - 1) / groups;
+        const long long most = dram ? kBuildLinkCtas : 12 * kBuildSms;
+        if (ctas > most) ctas = most;
+        build_pages_vec_kernel<T><<<(unsigned)ctas, kBuildThreads, 0, stream>>>(
+            static_cast<const unsigned char *>(k), static_cast<const unsigned char *>(v), tok_stride * E,
+            head_stride * E, static_cast<uint4 *>(dram), static_cast<uint4 *>(summaries), static_cast<uint4 *>(slots),
+            n_kv_heads, n_pages, n_slots, page_size, chunks);
+        return cudaGetLastError();
+    }
     int threads = head_dim < 32 ? 32 : (head_dim > 256 ? 256 : (head_dim + 31) / 32 * 32);
     dim3 grid(n_pages, n_kv_heads);
     build_pages_kernel<T><<<grid, threads, 0, stream>>>(

@@ -63,6 +63,7 @@ class DRAMAttention(torch.nn.Module):
         self._side = None
         self._fork_handle = None
         self._prefill_status = None
+        self._beside_construction = None
 
     # stage="prefill": this package's tcgen05 kernel where it applies (16-bit, head_dim 128)
     prefill_kernel = True
@@ -91,29 +92,32 @@ class DRAMAttention(torch.nn.Module):
         window (dram_attention/dram_attention.py:65-105)."""
         bsz, seqlen, H, D = k_cache.shape
         assert bsz == 1, "Only support batch size 1"
-        dram_kv_cache_size = seqlen - self.local_cache_size + self.page_size
-        self.dram_kv_cache_size = dram_kv_cache_size // self.page_size * self.page_size
-        L = seqlen - self.dram_kv_cache_size
-        self.cache_k[:, :L].copy_(k_cache[:, self.dram_kv_cache_size:], non_blocking=True)
-        self.cache_v[:, :L].copy_(v_cache[:, self.dram_kv_cache_size:], non_blocking=True)
-
-        dram_k_cache = k_cache[:, :self.dram_kv_cache_size]
-        dram_v_cache = v_cache[:, :self.dram_kv_cache_size]
-        if self.dram_kv_cache_size > self.lru_hbm_cache_size:
-            self.lru_cache = LRUCache(
+        beside, self._beside_construction = self._beside_construction, None
+        dram_kv_cache_size = (seqlen - self.local_cache_size + self.page_size) // self.page_size * self.page_size
+        dram_k_cache = k_cache[:, :dram_kv_cache_size]
+        dram_v_cache = v_cache[:, :dram_kv_cache_size]
+        if dram_kv_cache_size > self.lru_hbm_cache_size:
+            lru_cache = LRUCache(
                 k_cache=dram_k_cache[0].transpose(0, 1), v_cache=dram_v_cache[0].transpose(0, 1),
                 page_size=self.page_size, top_k=self.top_k // self.page_size,
-                lru_hbm_cache_size=self.lru_hbm_cache_size, device=self.device)
+                lru_hbm_cache_size=self.lru_hbm_cache_size, device=self.device, _beside=beside)
             # the kernel that fetches on the fly needs its 16-token units inside one page
             self._can_fuse = self.page_size % 16 == 0
             self._can_overlap = self._can_fuse   # refined per GQA group size at the first generate call
             self._overlap_ok = {}
         else:
-            self._can_fuse = False
-            self._can_overlap = False
-            self.lru_cache = DummyCache(
+            if beside is not None:
+                beside()
+            lru_cache = DummyCache(
                 k_cache=dram_k_cache[0].transpose(0, 1), v_cache=dram_v_cache[0].transpose(0, 1),
                 device=self.device, page_size=self.page_size)
+            self._can_fuse = False
+            self._can_overlap = False
+        self.lru_cache = lru_cache
+        self.dram_kv_cache_size = dram_kv_cache_size
+        L = seqlen - dram_kv_cache_size
+        self.cache_k[:, :L].copy_(k_cache[:, dram_kv_cache_size:], non_blocking=True)
+        self.cache_v[:, :L].copy_(v_cache[:, dram_kv_cache_size:], non_blocking=True)
 
     def init_cache_sharing(self, other: "DRAMAttention") -> None:
         """Initialise this operator as `init_cache` would with the prefill KV `other` was given,
@@ -152,9 +156,15 @@ class DRAMAttention(torch.nn.Module):
         if freqs_cis is not None:
             xq, xk = self.rotate_(xq, xk, freqs_cis)
         if stage == "prefill":
-            output = self._prefill_attention(xq, xk, xv)
-            self.init_cache(xk, xv)
-            return output
+            # the attention is enqueued from inside the construction of the cache, which fills the pinned pages over
+            # the host link while the tensor cores work (LRUCache's `_beside`)
+            outputs = []
+            self._beside_construction = lambda: outputs.append(self._prefill_attention(xq, xk, xv))
+            try:
+                self.init_cache(xk, xv)
+            finally:
+                self._beside_construction = None
+            return outputs[0] if outputs else self._prefill_attention(xq, xk, xv)
         elif stage == "generate":
             return self._generate(xq, xk, xv, start_pos)
         else:

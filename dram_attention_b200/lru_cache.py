@@ -64,7 +64,7 @@ class LRUCache(torch.nn.Module):
 
     def __init__(self, k_cache: torch.Tensor, v_cache: torch.Tensor, page_size: int, top_k: int,
                  lru_hbm_cache_size: Optional[int] = None, hbm_kv_cache_fraction: float = 0.2,
-                 device: str = "cuda", _share: Optional["LRUCache"] = None):
+                 device: str = "cuda", _share: Optional["LRUCache"] = None, _beside=None):
         super().__init__()
         if _share is not None:
             self._init_shared(_share, top_k)
@@ -89,31 +89,44 @@ class LRUCache(torch.nn.Module):
         k_dev, v_dev = k_cache.to(device=device), v_cache.to(device=device)
         _native.require_cuda(k_dev, "k_cache")
         dev = k_dev.device
-        i32 = dict(dtype=torch.int32, device=dev)
-        self.register_buffer("step_counters", torch.zeros(num_kv_heads, **i32))
-        self.register_buffer("dram_kv_cache", torch.empty(num_kv_heads, num_dram_pages, page_dim, dtype=dtype,
-                                                          device="cpu", pin_memory=True), persistent=False)
-        self.register_buffer("hbm_kv_cache", torch.empty(num_kv_heads, num_hbm_pages, page_dim, dtype=dtype,
-                                                         device=dev))
-        self.register_buffer("page_access_time", torch.zeros(num_kv_heads, num_hbm_pages, **i32))
-        # -1: the DRAM page is not in HBM; otherwise the slot that holds it
-        self.register_buffer("dram_page_to_hbm_page_mapping",
-                             torch.full((num_kv_heads, num_dram_pages), -1, **i32))
-        self.register_buffer("hbm_page_to_dram_page_mapping",
-                             torch.arange(num_dram_pages - num_hbm_pages, num_dram_pages, **i32)
-                             .repeat(num_kv_heads, 1))
-        # warm start: the rightmost pages are resident, slot s <- page Ld - Nh + s, times 0
-        self.dram_page_to_hbm_page_mapping[:, num_dram_pages - num_hbm_pages:] = \
-            torch.arange(num_hbm_pages, **i32)[None]
+        slots = torch.empty(num_kv_heads, num_hbm_pages, page_dim, dtype=dtype, device=dev)
         summaries = torch.empty(num_kv_heads, num_dram_pages, 2, head_dim, dtype=dtype, device=dev)
-        with torch.cuda.device(dev):
-            # one pass: pinned DRAM pages, page summaries and the resident slots
-            build_pages_(k_dev, v_dev, page_size, self.dram_kv_cache, summaries, self.hbm_kv_cache,
-                         num_hbm_pages)
-            torch.cuda.current_stream().synchronize()  # k_dev/v_dev may be temporaries
-        self.top_k_selector = IPUpperboundTopKSelector(k_cache, num_dram_pages, device=dev,
-                                                       _summaries=summaries)
-        self._init_tables(dev)
+        # One pass makes the pinned DRAM pages, the page summaries and the resident slots; the host link bounds it.
+        # `_beside` (a call that enqueues work on the current stream which neither needs nor touches the cache: the
+        # attention of the same prompt) runs at the same time: the pass then has a stream of its own, of high
+        # priority so that its few small CTAs find a place among the others', and waits only for what the
+        # current stream held before.  What it writes is allocated above, ahead of that wait: no memory that
+        # `_beside` gives back can be among it.
+        pages = torch.empty(num_kv_heads, num_dram_pages, page_dim, dtype=dtype, device="cpu", pin_memory=True)
+        stream = torch.cuda.current_stream(dev)
+        if _beside is not None:
+            main, stream = stream, torch.cuda.Stream(device=dev, priority=-1)
+            stream.wait_stream(main)
+        try:
+            with torch.cuda.device(dev), torch.cuda.stream(stream):
+                build_pages_(k_dev, v_dev, page_size, pages, summaries, slots, num_hbm_pages)
+            if _beside is not None:
+                _beside()
+            # the tables are set up while the pages are on their way
+            i32 = dict(dtype=torch.int32, device=dev)
+            self.register_buffer("step_counters", torch.zeros(num_kv_heads, **i32))
+            self.register_buffer("dram_kv_cache", pages, persistent=False)
+            self.register_buffer("hbm_kv_cache", slots)
+            self.register_buffer("page_access_time", torch.zeros(num_kv_heads, num_hbm_pages, **i32))
+            # -1: the DRAM page is not in HBM; otherwise the slot that holds it
+            self.register_buffer("dram_page_to_hbm_page_mapping",
+                                 torch.full((num_kv_heads, num_dram_pages), -1, **i32))
+            self.register_buffer("hbm_page_to_dram_page_mapping",
+                                 torch.arange(num_dram_pages - num_hbm_pages, num_dram_pages, **i32)
+                                 .repeat(num_kv_heads, 1))
+            # warm start: the rightmost pages are resident, slot s <- page Ld - Nh + s, times 0
+            self.dram_page_to_hbm_page_mapping[:, num_dram_pages - num_hbm_pages:] = \
+                torch.arange(num_hbm_pages, **i32)[None]
+            self.top_k_selector = IPUpperboundTopKSelector(k_cache, num_dram_pages, device=dev,
+                                                           _summaries=summaries)
+            self._init_tables(dev)
+        finally:
+            stream.synchronize()   # k_dev/v_dev may be temporaries, and the pages are in host memory from here on
 
     @classmethod
     def sharing_dram_of(cls, other: "LRUCache", top_k: Optional[int] = None) -> "LRUCache":

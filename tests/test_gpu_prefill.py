@@ -146,3 +146,30 @@ def test_prefill_kernel_heads_in_groups(da):
         sc = q[rows, h].double() @ k[:, h // 2].double().T / 128 ** 0.5
         ref = torch.softmax(sc.masked_fill(~seen, float("-inf")), -1) @ v[:, h // 2].double()
         _close(out[rows, h], ref, q.dtype)
+
+
+@pytest.mark.parametrize("lru", [1024, 8192])
+def test_prefill_builds_the_cache_beside_the_attention(da, lru):
+    """The pages, summaries and slots a prefill leaves (built while its attention runs) are those of init_cache, also
+    when the prompt's tensors are produced by work still in flight and given back right after the call."""
+    kw = dict(max_output_length=4, lru_hbm_cache_size=lru, local_cache_size=512, page_size=16, top_k=256, n_kv_heads=2,
+              head_dim=128)
+    g = torch.Generator(device=DEV).manual_seed(6)
+    s = 4500
+    q0, k0, v0 = (torch.randn(1, s, h, 128, generator=g, device=DEV).to(torch.bfloat16) for h in (8, 2, 2))
+    for _ in range(3):
+        a = da.DRAMAttention(device=DEV, dtype=torch.bfloat16, **kw)
+        b = da.DRAMAttention(device=DEV, dtype=torch.bfloat16, **kw)
+        torch.cuda._sleep(2_000_000)
+        q, k, v = q0 * 2, k0 * 2, v0 * 2
+        out = a(q, k, v, start_pos=0, stage="prefill")
+        del q, k, v
+        torch.full((1, s, 8, 128), float("nan"), dtype=torch.bfloat16, device=DEV)   # takes the memory over
+        b.init_cache(k0 * 2, v0 * 2)
+        assert torch.equal(a.cache_k[:, :500], b.cache_k[:, :500]) and torch.equal(a.cache_v[:, :500], b.cache_v[:, :500])
+        assert torch.equal(a.lru_cache.hbm_kv_cache, b.lru_cache.hbm_kv_cache)
+        if lru == 1024:
+            assert torch.equal(a.lru_cache.dram_kv_cache, b.lru_cache.dram_kv_cache)
+            assert torch.equal(a.lru_cache.top_k_selector.chunk_min_max, b.lru_cache.top_k_selector.chunk_min_max)
+        _close(out[0], _reference(q0[0] * 2, k0[0] * 2, v0[0] * 2), torch.bfloat16)
+        a.check_status()

@@ -735,3 +735,47 @@ def test_gather_wait_runs_out_and_is_reported(da):
                                0, status.data_ptr(), _native.stream_ptr()) == -2
     assert lib.da_gather_heads(local.data_ptr(), 24, ptrs.data_ptr(), seq.data_ptr(), 0, world, out.data_ptr(),
                                0, status.data_ptr(), _native.stream_ptr()) == -2
+
+
+# ------------------------------------------------------------------ cache construction ----
+
+@pytest.mark.parametrize("hk,tokens,page,d,dtype,offset,extra", [
+    (3, 60, 1, 128, torch.bfloat16, 0, 0),      # one token per page
+    (8, 176, 16, 128, torch.bfloat16, 0, 0),
+    (5, 99, 3, 64, torch.float16, 0, 0),        # groups that do not fill a CTA, a remainder of the unrolled loads
+    (2, 180, 18, 128, torch.float32, 0, 0),     # 64 threads per page
+    (1, 96, 32, 40, torch.bfloat16, 0, 0),      # 10 threads per page
+    (2, 64, 16, 264, torch.float32, 0, 0),      # rows longer than the 16-byte form takes
+    (2, 64, 16, 128, torch.bfloat16, 1, 0),     # rows off the 16-byte boundary
+    (2, 64, 16, 12, torch.float16, 0, 4),       # rows of 24 bytes
+])
+def test_build_pages_bytes(da, hk, tokens, page, d, dtype, offset, extra):
+    """Pages, resident slots and summaries, byte for byte, from strided keys and values with zeros of both signs,
+    infinities and NaN (a NaN that comes first in its page stays, a later one is passed over)."""
+    from dram_attention_b200.topk_selector import build_pages_
+    n_pages, n_slots = tokens // page, max(1, tokens // page // 3)
+    raw = torch.randn(2, tokens * hk * (d + extra) + offset, generator=_g(tokens + d)).to(dtype)
+    pick = torch.randint(0, 40, raw.shape, generator=_g(1))
+    for code, value in enumerate((0.0, -0.0, float("inf"), float("-inf"), float("nan"))):
+        raw[pick == code] = value
+    k, v = (r[offset:].view(tokens, hk, d + extra)[..., :d].transpose(0, 1) for r in raw)
+    dev = raw.to(DEV)
+    kd, vd = (r[offset:].view(tokens, hk, d + extra)[..., :d].transpose(0, 1) for r in dev)
+    dram = torch.empty(hk, n_pages, page, 2, d, dtype=dtype, pin_memory=True)
+    summaries = torch.empty(hk, n_pages, 2, d, dtype=dtype, device=DEV)
+    slots = torch.empty(hk, n_slots, page, 2, d, dtype=dtype, device=DEV)
+    build_pages_(kd, vd, page, dram, summaries, slots, n_slots)
+    alone = torch.empty_like(summaries)
+    build_pages_(kd, kd, page, None, alone, None, 0)
+    torch.cuda.synchronize()
+    bits = torch.int32 if dtype == torch.float32 else torch.int16
+    paged = torch.stack([k.reshape(hk, n_pages, page, d), v.reshape(hk, n_pages, page, d)], 3)
+    assert torch.equal(dram.view(bits), paged.view(bits))
+    assert torch.equal(slots.cpu().view(bits), paged[:, n_pages - n_slots:].contiguous().view(bits))
+    want = paged[:, :, 0, 0].clone().unsqueeze(2).repeat(1, 1, 2, 1)
+    for t in range(1, page):
+        key = paged[:, :, t, 0]
+        want[:, :, 0] = torch.where(key.float() < want[:, :, 0].float(), key, want[:, :, 0])
+        want[:, :, 1] = torch.where(key.float() > want[:, :, 1].float(), key, want[:, :, 1])
+    assert torch.equal(summaries.cpu().view(bits), want.view(bits))
+    assert torch.equal(alone.cpu().view(bits), want.view(bits))
