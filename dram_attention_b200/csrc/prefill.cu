@@ -19,13 +19,15 @@
 //
 // What bounds it: a CTA's chain is serial (S, softmax, product), since S, P and O fill its half of tensor memory, and
 // only the other CTA on the SM works meanwhile.  A tile needs the tensor core and the special-function unit for
-// 1024 cycles each, and takes 1840 (both are busy a little over half of the time).  128-key tiles, because every MMA
+// 1024 cycles each, and takes 1640 (both are busy five eighths of the time).  128-key tiles, because every MMA
 // of S reads its 4 KB slice of Q again: with 64 keys it moved 6 KB of shared memory for 32 cycles of
 // arithmetic.  K and V need one stage each: a key tile is refilled during the softmax, a value tile during the
 // next S and softmax.  Two threads per row, because one needs 168 registers for its 128 logits and leaves the
 // compiler no room to interleave (2.4 cycles of fixed latency per instruction); two need 96.
 // us for 2999 / 8192 / 16384 tokens x 32 heads: 64-key tiles, four softmax warps 129 / 591 / 2068; 128-key tiles
-// 104 / 512 / 1936; with eight softmax warps 100 / 492 / 1866 (1180 TFLOP/s).
+// 104 / 512 / 1936; with eight softmax warps 100 / 492 / 1866; with elect_one() below 95 / 467 / 1765 (1250 TFLOP/s; the SM
+// clock settles at 1.66 GHz).  Tried and slower: a quarter of the exponentials as polynomials on the multiply-add pipe
+// (2050), exponentials on the last tile's reference before the maximum is known (1835 to 1890).
 //
 // O never leaves tensor memory until the end: the exponentials of a row are taken against a
 // reference that follows the row maximum lazily, and O is rescaled in place (tcgen05.ld / st)
@@ -253,6 +255,16 @@ __device__ __forceinline__ uint32_t pack16(float lo, float hi) {
     return *reinterpret_cast<uint32_t *>(&v);
 }
 
+// True in one lane of a converged warp.  The compiler knows that nobody else is active behind it and keeps the operands
+// of the tensor-core and copy instructions, which live in registers of the warp, there; behind a comparison of the
+// lane number it moves them over for every instruction (16384 tokens x 32 heads: 1850 us, with this and a warp number
+// that is uniform to the compiler 1765).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+
 template <bool BF16>
 __global__ void __launch_bounds__(kPfThreads, 2)
 prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -269,7 +281,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     __shared__ int sh_abort;
 
     const int tid = threadIdx.x;
-    const int warp = tid >> 5;
+    const int warp = __shfl_sync(DA_FULL_MASK, tid >> 5, 0);
     // Within a group of heads the tiles with the most keys start first, so that what is left for the end of
     // the launch are the short ones.
     int qt, hq;
@@ -315,7 +327,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     if (warp == kPfSoftmaxWarps + 1) {
         // =================== the copy warp: every TMA copy, by one lane ===================================
         // Key tile j+1 goes where tile j was once S(j) is complete, value tile j+1 once the product of tile j is.
-        if ((tid & 31) == 0) {
+        if (elect_one()) {
             auto load_tile = [&](unsigned char *dst, const CUtensorMap *map, int j, uint64_t *bar) {
                 mbar_arrive_expect_tx(bar, kPfTileBytes);
                 tma_load_3d(dst, map, 0, hk, j * kPfKeys, bar);
@@ -342,7 +354,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         // =================== the issuing warp: every MMA, by one lane =====================================
         // Everything that can be is computed before the loop: the operand descriptors (an MMA's own is a
         // 64-bit add away).
-        if ((tid & 31) == 0) {
+        if (elect_one()) {
             const uint32_t idesc_s = instr_desc(bf16, false, kPfKeys), idesc_o = instr_desc(bf16, true, kPfDim);
             const uint64_t dq = desc_k_major(smem_addr(sQ)), dk = desc_k_major(smem_addr(sK));
             const uint64_t dv = desc_mn_major(smem_addr(sV));
@@ -366,8 +378,9 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 const uint32_t use = (uint32_t)(j & 1);
                 if (*abort_flag) break;
                 // O += P(j) V(j) once every softmax warp has written its part of P (and has rescaled its part of O
-                // if it had to)
-                ok = mbar_wait_bounded(&bar_v, use) && mbar_wait_bounded(&bar_p, use);
+                // if it had to); K(j+1) is waited for ahead of that, so that S(j+1) follows without a stop
+                ok = mbar_wait_bounded(&bar_v, use) && (j + 1 == n_tiles || mbar_wait_bounded(&bar_k, use ^ 1u)) &&
+                     mbar_wait_bounded(&bar_p, use);
                 if (!ok) break;
                 tc_fence_after();
                 if (j == 0) tc_mma_a_tmem_c<false>(tmem + tmem_o, tmem, dv, idesc_o);
@@ -377,11 +390,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     tc_mma_a_tmem_c<true>(tmem + tmem_o, tmem + (ks >> 2) * (kPfKeys / 2) + (ks & 3) * 8,
                                           dv + ((ks * 16 * 128) >> 4), idesc_o);
                 tc_commit(&bar_pv);
-                if (j + 1 < n_tiles) {
-                    ok = mbar_wait_bounded(&bar_k, use ^ 1u);
-                    if (!ok) break;
-                    issue_s();
-                }
+                if (j + 1 < n_tiles) issue_s();
             }
             if (!ok) give_up();
         }
