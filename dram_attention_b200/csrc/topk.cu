@@ -1,7 +1,7 @@
 // Per-query-head top-k page selection: radix select on order-preserving 32-bit
 // keys, exact lowest-index tie-break, then the k survivors are ranked by
-// (score descending, page id ascending).  One CTA per (token, query head) row, or a cluster of
-// four CTAs for rows of more than 16 384 pages; the result is written straight into the
+// (score descending, page id ascending).  One CTA per (token, query head) row (a cluster of
+// four for rows of more than 16 384 pages with a large k); the result is written straight into the
 // per-KV-head page list.
 
 #include "da_common.cuh"
@@ -438,7 +438,7 @@ topk_pages_kernel(const float *__restrict__ scores, int32_t *__restrict__ page_l
                   row_destination(page_list, row, gridDim.x, n_kv_heads, rep, k), smem_raw);
 }
 
-// ---- long rows: one row per cluster of kTopkCluster CTAs ---------------------------------------
+// ---- long rows with a large k: one row per cluster of kTopkCluster CTAs ---------------------------------------
 // A single CTA spends its time walking the row (64 keys per thread at 65 536 pages, several
 // sweeps).  Here every CTA of a cluster keeps a quarter of the row in registers (16 keys per
 // thread); the row's value range and the bucket counts are summed over the cluster through
@@ -653,6 +653,231 @@ topk_pages_cluster_kernel(const float *__restrict__ scores, int32_t *__restrict_
     }
     rank_candidates(cand, rank, lin_m, k, dst, tid);
 }
+// ---- long rows: one row per CTA, by the maxima of groups ----------------------------------------
+// A row of 65 536 scores does not fit a CTA's registers, and several sweeps over it cost 38 us.  Here it is read
+// once: a thread keeps the maxima of kGroups groups of 4 * PER scores.  The k-th largest of all group maxima is a
+// lower bound of the k-th largest score (k groups hold at least one score each that reaches it), so the
+// selected pages lie in the groups whose maximum reaches the bucket of that bound: a few more than k of them, which
+// are read a second time.  Bound by latency: 2.5 us for the row out of L2, then five dependent stages.  Their scores from that bucket on are the candidates, sorted by bucket and
+// ranked inside their bucket as in the kernel above.  Rows this cannot resolve (NaN, constant rows, massive
+// ties) fall back to the one-CTA selection.  The scores stay in L2 between the two readings.
+constexpr int kGroups = 8;
+constexpr int kGroupElems = 8;      // scores of qualifying groups a thread can hold
+__host__ __device__ inline bool topk_groups_fit(int n_pages, int per, int k) {
+    return n_pages <= kGroups * per * 4 * kTopkThreads && topk_candidate_capacity(k) * 4 * per <= kGroupElems * kTopkThreads;
+}
+
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// VEC: the row starts on a 16-byte boundary and its length is a multiple of 4; four consecutive scores per load.
+// Otherwise four coalesced loads.  Score q of load `it` of thread t:
+template <bool VEC> __device__ __forceinline__ int group_element(int it, int q, int t) {
+    return VEC ? 4 * (it * kTopkThreads + t) + q : (it * 4 + q) * kTopkThreads + t;
+}
+
+template <int PER, bool VEC>
+__global__ void __launch_bounds__(kTopkThreads)
+topk_pages_groups_kernel(const float *__restrict__ scores, int32_t *__restrict__ page_list, int n_kv_heads, int rep,
+                         int n_pages, int k) {
+    if (threadIdx.x == 0) trace_stamp(1, blockIdx.x, 0);
+    struct EndStamp {
+        __device__ ~EndStamp() {
+            if (threadIdx.x == 0) trace_stamp(1, blockIdx.x, 1);
+        }
+    } end_stamp;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int cap = topk_candidate_capacity(k);
+    unsigned long long *cand = reinterpret_cast<unsigned long long *>(smem_raw);  // [cap + 2]
+    int *groups = reinterpret_cast<int *>(cand + cap + 2);                        // [cap] groups to read again
+    __shared__ int hist[2][256];      // group maxima per bucket, levels 1 and 2
+    __shared__ int count_of[256];     // candidates per bucket
+    __shared__ int above_of[256];     // candidates in higher buckets
+    __shared__ int fill[256];         // places handed out per bucket
+    __shared__ uint32_t sh_kmin, sh_kmax;
+    __shared__ int sh_digit, sh_above, sh_count, sh_groups;
+
+    const int tid = threadIdx.x;
+    const int lane = tid & 31;
+    const int warp = tid >> 5;
+    const int row = blockIdx.x;
+    const float *srow = scores + (size_t)row * n_pages;
+    int32_t *dst = row_destination(page_list, row, gridDim.x, n_kv_heads, rep, k);
+
+    if (tid < 256) {
+        hist[0][tid] = 0;
+        hist[1][tid] = 0;
+        count_of[tid] = 0;
+        fill[tid] = 0;
+    }
+    if (tid == 0) {
+        sh_kmin = 0xffffffffu;
+        sh_kmax = 0u;
+        sh_groups = 0;
+    }
+    griddep_wait();                // the scores come from the kernel before this one
+    if (tid == 0) trace_stamp(1, blockIdx.x, 2);
+    griddep_launch_dependents();   // the LRU update may move onto the SMs and wait there
+
+    // ---- the maxima: 32 scores per thread in flight ---------------------------------------------
+    constexpr int kBatch = 8 / PER;         // groups per batch of 8 loads
+    float gm[kGroups];
+#pragma unroll
+    for (int g0 = 0; g0 < kGroups; g0 += kBatch) {
+        float v[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int it = g0 * PER + i;
+            if constexpr (VEC) {
+                const int e = group_element<true>(it, 0, tid);
+                const float4 x = e < n_pages ? *reinterpret_cast<const float4 *>(srow + e)
+                                             : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+                v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int e = group_element<false>(it, q, tid);
+                    v[i][q] = e < n_pages ? srow[e] : -INFINITY;
+                }
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < kBatch; ++g) {
+            float m = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < PER; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) m = max_nan(m, v[g * PER + i][q]);
+            gm[g0 + g] = m;
+        }
+    }
+    auto live = [&](int g) { return group_element<VEC>(g * PER, 0, tid) < n_pages; };
+
+    // ---- bucket of the k-th largest group maximum ------------------------------------------------
+    uint32_t kmn = 0xffffffffu, kmx = 0u;
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g) {
+        if (live(g)) {
+            const uint32_t key = score_key(gm[g]);
+            kmn = min(kmn, key);
+            kmx = max(kmx, key);
+        }
+    }
+    kmn = __reduce_min_sync(DA_FULL_MASK, kmn);
+    kmx = __reduce_max_sync(DA_FULL_MASK, kmx);
+    __syncthreads();
+    if (lane == 0) {
+        atomicMin(&sh_kmin, kmn);
+        atomicMax(&sh_kmax, kmx);
+    }
+    __syncthreads();
+    const float lo = key_score(sh_kmin), hi = key_score(sh_kmax);
+    const float width = hi - lo;
+    if (!(width > 0.f && width < 3.0e38f)) {   // also NaN; uniform
+        topk_row_fallback(srow, n_pages, k, dst, smem_raw);
+        return;
+    }
+    const float lin_scale = 256.f / width;
+    float lo2 = 0.f, scale2 = 0.f;
+    int b1 = 0, b2 = 0, levels = 0, n_groups = 0;
+    {
+        int need = k, above_total = 0;
+        for (int level = 1; level <= 2; ++level) {
+            int *h = hist[level - 1];
+#pragma unroll
+            for (int g = 0; g < kGroups; ++g) {
+                if (!live(g)) continue;
+                const int b = linear_bucket(gm[g], lo, lin_scale);
+                if (level == 1) atomicAdd(&h[b], 1);
+                else if (b == b1) atomicAdd(&h[linear_bucket(gm[g], lo2, scale2)], 1);
+            }
+            __syncthreads();
+            if (warp == 0) descending_crossing(h, need, lane, &sh_digit, &sh_above, &sh_count);
+            __syncthreads();
+            const int b = sh_digit, above = sh_above;
+            n_groups = above_total + above + sh_count;
+            levels = level;
+            if (level == 1) {
+                b1 = b;
+                lo2 = lo + (float)b / lin_scale;
+                scale2 = lin_scale * 256.f;
+            } else {
+                b2 = b;
+            }
+            above_total += above;
+            need -= above;
+            if (n_groups <= k + (k >> 2)) break;    // room for the groups that hold more than one candidate
+            __syncthreads();   // sh_* are rewritten by the next level
+        }
+    }
+    if (n_groups > cap) {
+        __syncthreads();
+        topk_row_fallback(srow, n_pages, k, dst, smem_raw);
+        return;
+    }
+    auto reaches = [&](float x) {
+        const int b = linear_bucket(x, lo, lin_scale);
+        if (levels == 1 || b != b1) return b >= b1;
+        return linear_bucket(x, lo2, scale2) >= b2;
+    };
+
+    // ---- those groups' scores again, the candidates among them counted per bucket -----------------------
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g)
+        if (live(g) && reaches(gm[g])) groups[atomicAdd(&sh_groups, 1)] = g * kTopkThreads + tid;
+    __syncthreads();
+    const int n_elems = n_groups * 4 * PER;      // <= kGroupElems * kTopkThreads (see topk_groups_fit)
+    float x[kGroupElems];
+    int id[kGroupElems];
+#pragma unroll
+    for (int i = 0; i < kGroupElems; ++i) {
+        const int at = i * kTopkThreads + tid;
+        id[i] = -1;
+        if (at < n_elems) {
+            const int grp = groups[at / (4 * PER)], w = at % (4 * PER);
+            const int e = group_element<VEC>(grp / kTopkThreads * PER + w / 4, w % 4, grp % kTopkThreads);
+            if (e < n_pages) {
+                x[i] = srow[e];
+                id[i] = e;
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kGroupElems; ++i) {
+        if (id[i] >= 0 && reaches(x[i])) atomicAdd(&count_of[linear_bucket(x[i], lo, lin_scale)], 1);
+        else id[i] = -1;
+    }
+    __syncthreads();
+    if (warp == 0) descending_crossing(count_of, k, lane, &sh_digit, &sh_above, &sh_count, above_of);
+    __syncthreads();
+    const int m = above_of[b1] + count_of[b1];   // every candidate: no bucket below b1 has any
+    if (m > cap) {
+        __syncthreads();
+        topk_row_fallback(srow, n_pages, k, dst, smem_raw);
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < kGroupElems; ++i) {
+        if (id[i] < 0) continue;
+        const int b = linear_bucket(x[i], lo, lin_scale);
+        cand[above_of[b] + atomicAdd(&fill[b], 1)] =
+            ((unsigned long long)(~score_key(x[i])) << 32) | (uint32_t)id[i];
+    }
+    __syncthreads();
+    for (int e = tid; e < m; e += kTopkThreads) {
+        const unsigned long long v = cand[e];
+        const int b = linear_bucket(key_score(~(uint32_t)(v >> 32)), lo, lin_scale);
+        const int first = above_of[b];
+        const int last = first + count_of[b];
+        int c = first;
+        for (int j = first; j < last; ++j) c += cand[j] < v;
+        if (c < k) dst[c] = (int32_t)(v & 0xffffffffu);
+    }
+}
+
 template <int IPT>
 static cudaError_t launch_topk(const float *scores, int32_t *page_list, int rows, int n_kv_heads, int rep,
                                int n_pages, int k, cudaStream_t stream) {
@@ -674,6 +899,24 @@ static cudaError_t launch_topk(const float *scores, int32_t *page_list, int rows
                                             scores, page_list, n_kv_heads, rep, n_pages, k);
     if (le != cudaSuccess) return le;
     return cudaGetLastError();
+}
+
+template <int PER, bool VEC>
+static cudaError_t launch_topk_groups(const float *scores, int32_t *page_list, int rows, int n_kv_heads, int rep,
+                                      int n_pages, int k, cudaStream_t stream) {
+    const int cap = topk_candidate_capacity(k);      // at most 2048 here: 24 KB, no opt-in needed
+    const size_t smem = (size_t)(cap + 2) * sizeof(unsigned long long) + (size_t)cap * sizeof(int);
+    const cudaError_t e = launch_dependent(topk_pages_groups_kernel<PER, VEC>, dim3(rows), dim3(kTopkThreads), smem, stream,
+                                           scores, page_list, n_kv_heads, rep, n_pages, k);
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+template <int PER>
+static cudaError_t launch_topk_groups(const float *scores, int32_t *page_list, int rows, int n_kv_heads, int rep,
+                                      int n_pages, int k, cudaStream_t stream) {
+    if (n_pages % 4 == 0 && ((uintptr_t)scores & 15) == 0)
+        return launch_topk_groups<PER, true>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, stream);
+    return launch_topk_groups<PER, false>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, stream);
 }
 
 static cudaError_t launch_topk_cluster(const float *scores, int32_t *page_list, int rows, int n_kv_heads, int rep,
@@ -721,13 +964,19 @@ extern "C" int da_topk_pages_wide(const float *scores, int32_t *page_list, int n
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaError_t e;
     if (sm_budget == 0) sm_budget = 148;
-    // long rows are split over a cluster when all clusters find an SM per CTA at once; otherwise the
-    // clusters would run in turns and one CTA per row is as fast
-    if (n_pages > 16 * da::kTopkThreads && n_pages <= da::kTopkClusterMaxPages && rows * da::kTopkCluster <= sm_budget)
-        e = da::launch_topk_cluster(scores, page_list, rows, n_kv_heads, rep, n_pages, k, s);
-    else if (n_pages <= 4 * da::kTopkThreads) e = da::launch_topk<4>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, s);
+    // Rows that fit the registers of a CTA are selected from there.  Longer ones by the maxima of groups, as long as k
+    // leaves the groups to be read again few; with a larger k they are split over a cluster when all clusters find an
+    // SM per CTA at once (otherwise the clusters would run in turns), and swept by one CTA at last.  us for
+    // 32 rows of 65 536 pages, k = 256: groups 8.6, clusters 10.4, sweeps 38; 20 000 pages: 7.1, 9.4.
+    const bool long_row = n_pages > 16 * da::kTopkThreads;
+    if (n_pages <= 4 * da::kTopkThreads) e = da::launch_topk<4>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, s);
     else if (n_pages <= 8 * da::kTopkThreads) e = da::launch_topk<8>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, s);
-    else if (n_pages <= 16 * da::kTopkThreads) e = da::launch_topk<16>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, s);
+    else if (!long_row) e = da::launch_topk<16>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, s);
+    else if (da::topk_groups_fit(n_pages, 1, k)) e = da::launch_topk_groups<1>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, s);
+    else if (da::topk_groups_fit(n_pages, 2, k)) e = da::launch_topk_groups<2>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, s);
+    else if (da::topk_groups_fit(n_pages, 4, k)) e = da::launch_topk_groups<4>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, s);
+    else if (n_pages <= da::kTopkClusterMaxPages && rows * da::kTopkCluster <= sm_budget)
+        e = da::launch_topk_cluster(scores, page_list, rows, n_kv_heads, rep, n_pages, k, s);
     else e = da::launch_topk<0>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, s);
     return (int)e;
 }

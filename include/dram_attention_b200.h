@@ -125,10 +125,10 @@ DA_API int da_topk_pages(const float *scores, int32_t *page_list,
                   da_stream_t stream);
 
 /*
- * The same selection with a hint on how many SMs it may count on.  Rows of more than 16 384 pages
- * (up to 65 536) are split over a thread-block cluster of four CTAs (partial histograms summed
- * through distributed shared memory, candidates collected in one CTA) when all clusters of the
- * launch find an SM per CTA at once: n_tokens * n_kv_heads * rep * 4 <= sm_budget.  A caller
+ * The same selection with a hint on how many SMs it may count on.  Rows of 16 385 to 65 536
+ * pages with a large k (above 682 to 1365, by their length) are split over a thread-block cluster of four CTAs (partial
+ * histograms summed through distributed shared memory, candidates collected in one CTA) when all
+ * clusters of the launch find an SM per CTA at once: n_tokens * n_kv_heads * rep * 4 <= sm_budget.  A caller
  * that runs another launch beside the selection (the first attention launch of the two-launch
  * step keeps all but 32 SMs) passes what is left; 0 means the whole GPU, which is what
  * da_topk_pages passes.  The result does not depend on sm_budget.

@@ -779,3 +779,35 @@ def test_build_pages_bytes(da, hk, tokens, page, d, dtype, offset, extra):
         want[:, :, 1] = torch.where(key.float() > want[:, :, 1].float(), key, want[:, :, 1])
     assert torch.equal(summaries.cpu().view(bits), want.view(bits))
     assert torch.equal(alone.cpu().view(bits), want.view(bits))
+
+
+# ------------------------------------------------------------- selection of long rows, one CTA each ----
+
+@pytest.mark.parametrize("pages,k", [(16385, 1), (16388, 1365), (16388, 1366), (32768, 300), (32769, 300), (32772, 682), (32772, 683),
+                                     (65535, 256), (65536, 682), (65537, 200), (65540, 341), (65540, 342), (131072, 100),
+                                     (131075, 256)])
+@pytest.mark.parametrize("kind", ["normal", "needles", "quantised", "outlier", "nan", "inf", "falling"])
+def test_topk_long_rows_by_group_maxima(da, pages, k, kind):
+    """Selection with one SM to count on, at both sides of every size at which the number of scores per group changes
+    or the group path ends, against a stable descending sort of the same order (NaN above everything)."""
+    from dram_attention_b200 import _native
+    g = _g(pages + k)
+    sc = torch.randn(2, pages, generator=g) * 30
+    if kind == "needles":
+        sc[:, torch.randperm(pages, generator=g)[:32]] += 900.0      # leaves the rest of the row to a few buckets
+    elif kind == "quantised":
+        sc = torch.round(sc / 8)
+    elif kind == "outlier":
+        sc[:, 5], sc[:, 77] = 1e30, -1e30
+    elif kind == "nan":
+        sc[0, pages // 2] = float("nan")
+    elif kind == "inf":
+        sc[0, 3], sc[1, pages - 1] = float("inf"), float("-inf")
+    elif kind == "falling":
+        sc = sc.sort(-1, descending=True).values                     # the best scores side by side
+    dev = sc.to(DEV)
+    out = torch.full((1, 2 * k), -7, dtype=torch.int32, device=DEV)
+    _native.check(_native.lib().da_topk_pages_wide(dev.data_ptr(), out.data_ptr(), 1, 1, 2, pages, k, 1,
+                                                   _native.stream_ptr()))
+    want = torch.sort(sc, dim=-1, descending=True, stable=True).indices[:, :k].reshape(1, -1).to(torch.int32)
+    assert torch.equal(out.cpu(), want)
