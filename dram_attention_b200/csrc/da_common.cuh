@@ -226,6 +226,11 @@ __device__ __forceinline__ void bulk_copy_g2s(void *dst_smem, const void *src_gm
 }
 
 
+// Brings `bytes` at `src` into L2 (address and size multiples of 16).
+__device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
 // Same, with an L2 eviction-priority hint for the lines it brings in.  Streaming reads that
 // nobody will touch again soon should be marked evict-first so that they do not push small,
 // latency-critical data (scores, tables) of concurrently running kernels out of L2.
