@@ -24,6 +24,18 @@ namespace da {
 // 85.8 / 81.4 / 79.0 / 81.2 us, four 128K layers 168.3 / 166.4 / 166.6 / 171.3).
 constexpr int kPrefetchUnits = 2;
 
+// The ticket word of a head, zero between two steps.
+constexpr unsigned int kTicketPhase2 = 1u << 12;     // a CTA of phase 2 (a launch has at most kAttnMaxSplits per head)
+constexpr unsigned int kTicketMerged = 1u << 30;     // phase 1's partials have been merged into one
+static_assert(kAttnMaxSplits < (int)kTicketPhase2, "the counts of the two launches stay apart");
+enum { kMergeNothing, kMergePhase1, kMergeAll, kMergeRest };
+
+__device__ __forceinline__ unsigned int take_ticket(unsigned int *word, unsigned int add) {
+    unsigned int old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(word), "r"(add) : "memory");
+    return old;
+}
+
 template <typename Math, int WARPS, int STAGES>
 __device__ __forceinline__ void decode_attention_body(const AttnParams &p, unsigned char *smem) {
     using T = typename Math::Elem;
@@ -40,7 +52,7 @@ __device__ __forceinline__ void decode_attention_body(const AttnParams &p, unsig
 
     __shared__ __align__(8) uint64_t bars[WARPS][STAGES];
     __shared__ __align__(16) uint4 plan_tab[WARPS][kRoundUnits];
-    __shared__ int sh_last;
+    __shared__ int sh_merge;
 
     const int h = blockIdx.y;
     const int x = blockIdx.x;
@@ -86,6 +98,11 @@ __device__ __forceinline__ void decode_attention_body(const AttnParams &p, unsig
     //      one round trip to memory instead of one after the other ------------------------------------
     const int pos = p.start_pos_dev ? *p.start_pos_dev : p.start_pos_host;
     const FrontWords fw = load_front(p, h);
+    const int n_workers = splits * WARPS;
+    // warp-major worker ids: the workers that get one unit more than the others are spread over all CTAs of
+    // the head (one or two per SM), not packed into the first CTAs (twelve on the same SM)
+    const int worker = warp * splits + x;
+    const FirstSlots fs = load_first_slots(p, h, worker, n_workers, lane);
     typename Math::State st;
     Math::init(st, p, h, lane, rows);
 
@@ -99,10 +116,6 @@ __device__ __forceinline__ void decode_attention_body(const AttnParams &p, unsig
     }
     const int n_local = t0 + p.s_total;
     const int n_prefix = p.n_prefix_tokens;
-    const int n_workers = splits * WARPS;
-    // warp-major worker ids: the workers that get one unit more than the others are spread over all CTAs of
-    // the head (one or two per SM), not packed into the first CTAs (twelve on the same SM)
-    const int worker = warp * splits + x;
     LaunchUnits lu = launch_units(p, h, n_local, false, fw);
     int units = lu.units_slots + lu.units_local;
     int total_my = units > worker ? (units - worker + n_workers - 1) / n_workers : 0;
@@ -129,22 +142,27 @@ __device__ __forceinline__ void decode_attention_body(const AttnParams &p, unsig
     const uint64_t stream_policy = l2_policy_evict_first();   // the KV stream is read once per step
     bool dead = false;
 
-    int base0 = plan_base(p, lu, worker, n_workers, lane, 0, total_my);
+    int base0 = plan_base(p, lu, worker, n_workers, lane, 0, total_my, (fw.flip & 1) ? fs.copy1 : fs.copy0);
     if (p.phase == 2) {
         griddep_wait();   // from here on the LRU update is complete
         griddep_launch_dependents();
+    }
+    int src0 = plan_source(p, h, base0);   // (set out together with the redo flag)
+    if (p.phase == 2) {
         if (p.redo[h] != 0) {
             // it evicted beyond the front: this launch covers the whole head
             lu = launch_units(p, h, n_local, true, fw);
             units = lu.units_slots + lu.units_local;
             total_my = units > worker ? (units - worker + n_workers - 1) / n_workers : 0;
             base0 = plan_base(p, lu, worker, n_workers, lane, 0, total_my);
+            src0 = plan_source(p, h, base0);
         }
     }
 
     for (int round = 0; round * kRoundUnits < total_my && !dead; ++round) {
         const int base = round == 0 ? base0 : plan_base(p, lu, worker, n_workers, lane, round, total_my);
-        const int n_round = plan_commit(p, lu, h, worker, n_workers, lane, round, total_my, base, tab, (size_t)E);
+        const int src = round == 0 ? src0 : plan_source(p, h, base);
+        const int n_round = plan_commit(p, lu, h, worker, n_workers, lane, round, total_my, base, src, tab, (size_t)E);
         const int g0 = round * kRoundUnits;   // units this warp has consumed before this round
 
         // start the copies of the unit at position `it` of this round into stage s
@@ -270,23 +288,45 @@ __device__ __forceinline__ void decode_attention_body(const AttnParams &p, unsig
         // The ticket releases this CTA's rows (ordered before this thread by the barrier) and acquires the rows
         // of every CTA that took a ticket before: one acq_rel read-modify-write at GPU scope instead of a fence
         // on either side.  The barrier below carries the acquire to the other threads of the CTA.
-        unsigned int ticket;
-        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(p.counters + h) : "memory");
-        sh_last = (ticket == (unsigned int)(p.ticket_target - 1));
+        // The word counts the CTAs of phase 1 (and of a single launch) in its low bits and those of phase 2 above.
+        const unsigned int old = take_ticket(p.counters + h, p.phase == 2 ? kTicketPhase2 : 1u);
+        const int done1 = (int)(old & (kTicketPhase2 - 1)), done2 = (int)((old & (kTicketMerged - 1)) / kTicketPhase2);
+        int todo = kMergeNothing;
+        if (done1 + done2 == p.ticket_target - 1) todo = (old & kTicketMerged) ? kMergeRest : kMergeAll;
+        else if (p.phase == 1 && done1 == p.splits1 - 1 && p.splits1 > 2) todo = kMergePhase1;
+        sh_merge = todo;
     }
     __syncthreads();
+    const int todo = sh_merge;
     if (tid == 0) {
         trace_stamp(trace_kernel, trace_cta, 3);
-        if (!sh_last) trace_stamp(trace_kernel, trace_cta, 1);
+        if (todo == kMergeNothing) trace_stamp(trace_kernel, trace_cta, 1);
     }
-    if (!sh_last) return;
+    if (todo == kMergeNothing) return;
+
+    if (todo == kMergePhase1) {
+        // ---- the last CTA of phase 1, phase 2 still at work: phase 1's partials become one, so that the merge at the
+        //      end of the step has only phase 2's few beside it (8 rows of 44 partials: 5.4 us, of 7: 3.1) ------
+        merge_partials<T, D, THREADS>(p, h, 0, p.splits1, rows, nullptr,
+                                      p.partials + ((size_t)(h * p.part_rows + p.ticket_target) * rows) * PW, smem);
+        __syncthreads();
+        if (tid == 0) {
+            // Said in the ticket word, where the last CTA reads it with its ticket.  A word that is zero again means
+            // that the last CTA is through, without it; nobody reads the word any more in this step.
+            if (take_ticket(p.counters + h, kTicketMerged) == 0u) take_ticket(p.counters + h, 0u - kTicketMerged);
+            trace_stamp(trace_kernel, trace_cta, 1);
+        }
+        return;
+    }
 
     // ---- the CTA of this head that finished last (of both launches, when there are two) --------
-    // a head that phase 2 redid: phase 1's rows (the first in the workspace) are left out
-    merge_splits<T, D, THREADS>(p, h, p.part_rows, rows, p.phase != 0 ? p.redo + h : nullptr, p.splits1, smem);
+    // a head that phase 2 redid: phase 1's rows (the first in the workspace, or merged into the one behind all) are left out
+    const bool rest = todo == kMergeRest;
+    merge_partials<T, D, THREADS>(p, h, rest ? p.splits1 : 0, p.ticket_target + (rest ? 1 : 0), rows,
+                                  p.phase != 0 ? p.redo + h : nullptr, nullptr, smem);
     // every CTA of this head is done with the eviction front: the one the LRU update left becomes current
     if (p.phase != 0 && tid == 0) atomicXor(p.flip + h, 1);   // (no result wanted: the CTA does not wait for it)
-    if (tid == 0) p.counters[h] = 0u;
+    if (tid == 0) asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p.counters + h), "r"(0u) : "memory");
     if (tid == 0) trace_stamp(trace_kernel, trace_cta, 1);
 }
 

@@ -99,7 +99,7 @@ struct AttnParams {
     const int32_t *n_evictable;      // [2][n_kv_heads]
     int32_t *flip;                   // [n_kv_heads]
     const int32_t *redo;             // [n_kv_heads]
-    int part_rows;                   // partial rows (CTAs) per head in the workspace
+    int part_rows;                   // partials per head in the workspace (two launches: one more than CTAs)
     int part_offset;                 // first row this launch writes
     int ticket_target;               // CTAs of a head that take a ticket before the merge
     int splits1;                     // rows of phase 1 (first in the workspace)
@@ -116,7 +116,6 @@ struct LaunchUnits {
     int units_slots;      // units from the slot table
     int units_local;      // units from the local window
     const int32_t *order; // slot order to walk (null: slot-table tokens in place)
-    int order_off;        // first entry of `order` that belongs to this launch
     int ups;              // units per slot page
 };
 
@@ -139,7 +138,6 @@ __device__ __forceinline__ LaunchUnits launch_units(const AttnParams &p, int h, 
                                                     const FrontWords &fw) {
     LaunchUnits lu;
     lu.order = nullptr;
-    lu.order_off = 0;
     lu.ups = p.phase != 0 ? p.page_tokens / kUnitTokens : 1;
     bool local = true;
     if (p.phase == 0) {
@@ -152,7 +150,6 @@ __device__ __forceinline__ LaunchUnits launch_units(const AttnParams &p, int h, 
         if (p.phase == 1) {
             lu.units_slots = (p.n_slots - n_ev) * lu.ups;
             lu.order = order;
-            lu.order_off = n_ev;
         } else if (redo) {
             lu.units_slots = p.n_slots * lu.ups;   // the whole head, slots in place
         } else {
@@ -175,16 +172,37 @@ __device__ __forceinline__ LaunchUnits launch_units(const AttnParams &p, int h, 
 // the LRU update has finished: plan_base() needs only the eviction queue as it was BEFORE the
 // update, plan_commit() the marks the update leaves (which slots must be read from DRAM).
 
-// First slot-table token of lane's unit of this round, or -1 (a local-window unit, or none).
+// Place in the eviction queue of the k-th slot a launch walks: phase 2 from the front, phase 1 from the back, so that
+// neither has to know how long the front is before it reads the queue.
+__device__ __forceinline__ int queue_place(const AttnParams &p, int k) { return p.phase == 1 ? p.n_slots - 1 - k : k; }
+
+// The slots of the first round's units out of both copies of the queue, read before it is known which one is current.
+struct FirstSlots {
+    int copy0, copy1;
+};
+__device__ __forceinline__ FirstSlots load_first_slots(const AttnParams &p, int h, int worker, int n_workers, int lane) {
+    FirstSlots f = {0, 0};
+    if (p.phase != 0) {
+        const int at = queue_place(p, (worker + lane * n_workers) / (p.page_tokens / kUnitTokens));
+        if (at >= 0 && at < p.n_slots) {
+            f.copy0 = p.order[(size_t)h * p.n_slots + at];
+            f.copy1 = p.order[((size_t)p.n_kv_heads + h) * p.n_slots + at];
+        }
+    }
+    return f;
+}
+
+// First slot-table token of lane's unit of this round, or -1 (a local-window unit, or none).  `first` (round 0): the
+// slot of that unit in the queue.
 __device__ __forceinline__ int plan_base(const AttnParams &p, const LaunchUnits &lu, int worker, int n_workers,
-                                         int lane, int round, int total_my) {
+                                         int lane, int round, int total_my, int first = 0) {
     const int n_round = min(kRoundUnits, total_my - round * kRoundUnits);
     const int u = worker + (round * kRoundUnits + lane) * n_workers;
     int base = -1;
     if (lane < n_round && u < lu.units_slots) {
         base = u * kUnitTokens;
         if (lu.order) {
-            int slot = lu.order[lu.order_off + u / lu.ups];
+            int slot = round == 0 ? first : lu.order[queue_place(p, u / lu.ups)];
             slot = min(max(slot, 0), p.n_slots - 1);
             base = slot * p.page_tokens + (u % lu.ups) * kUnitTokens;
         }
@@ -192,17 +210,20 @@ __device__ __forceinline__ int plan_base(const AttnParams &p, const LaunchUnits 
     return base;
 }
 
+// DRAM page lane's unit has to be read from, or -1.
+__device__ __forceinline__ int plan_source(const AttnParams &p, int h, int base) {
+    if (base < 0 || !p.slot_source || p.phase == 1) return -1;
+    return p.slot_source[(size_t)h * p.n_slots + base / p.page_tokens];
+}
+
 // Writes the round's table.  Units that have to come from DRAM are visited first, so that their
 // host-link latency overlaps everything else the warp does.  Returns n_round.
 __device__ __forceinline__ int plan_commit(const AttnParams &p, const LaunchUnits &lu, int h, int worker,
-                                           int n_workers, int lane, int round, int total_my, int base,
+                                           int n_workers, int lane, int round, int total_my, int base, int src,
                                            uint4 *tab, size_t elem_bytes) {
     const int n_round = min(kRoundUnits, total_my - round * kRoundUnits);
     const int u = worker + (round * kRoundUnits + lane) * n_workers;
     const bool valid = lane < n_round;
-    int src = -1;
-    if (base >= 0 && p.slot_source && p.phase != 1)
-        src = p.slot_source[(size_t)h * p.n_slots + base / p.page_tokens];
     const unsigned fresh = __ballot_sync(DA_FULL_MASK, valid && src >= 0);
     if (valid) {
         const int before = __popc(fresh & ((1u << lane) - 1));
@@ -250,24 +271,29 @@ __device__ __forceinline__ void merge_into(MergeAcc &x, float m, float l, const 
     x.a.w = x.a.w * wx + v.w * wv;
 }
 
-// Final merge of the per-CTA partials of one head by one CTA of THREADS threads.  A CTA's partial = `rows` rows
+// Merge of the per-CTA partials [lo, hi) of one head by one CTA of THREADS threads.  A CTA's partial = `rows` rows
 // of (acc[D] already weighted to the row's max, max, l); the partials of consecutive CTAs are contiguous in the
 // workspace.  It is on the critical path of every step and bound by latency alone, so it is one round trip to
 // L2 wherever the registers allow: a thread owns four columns of a row for every G-th CTA (G = how many
-// times the row-columns fit into the CTA), requests kMergeBatch partials together with their (max, l) pairs, and
+// times the row-columns fit into the CTA), requests BATCH partials together with their (max, l) pairs, and
 // folds them in registers; the G groups meet in shared memory.  (Staging the rows in shared memory in two
 // halves, as before, took one round trip per half: 3.7 us for 22 partials of 4 rows, 5.9 us for 55.)
-// `skip_flag` (may be null): when the word it points to is non-zero the first `skip` CTAs' rows are left out.
+// `merged` (may be null): where the result goes as one more partial; otherwise it is the head's output.
+// `skip_flag` (may be null): when the word it points to is non-zero phase 1's partials, and the one they were
+// merged into, are left out.
+// With kMergeBatchFew partials per thread or less a short batch: the long one asks for the last partial again and
+// again (four resident 13K layers 78.3 / 74.0 us).
 constexpr int kMergeBatch = 18;
+constexpr int kMergeBatchFew = 6;
 
-template <typename T, int D, int THREADS>
-__device__ __forceinline__ void merge_splits(const AttnParams &p, int h, int splits, int rows, const int32_t *skip_flag,
-                                             int skip, unsigned char *smem) {
+template <typename T, int D, int THREADS, int BATCH>
+__device__ __forceinline__ void merge_range(const AttnParams &p, int h, int lo, int hi, int rows, const int32_t *skip_flag,
+                                            float *merged, unsigned char *smem) {
     constexpr int PW = PartialRow<D>::kWidth;
     constexpr int VPR = D / 4;          // float4 per accumulator row
     const int tid = threadIdx.x;
     const int32_t peer_step = p.peer_world > 0 ? __ldcg(p.peer_seq) : 0;   // (needed at the very end: read now)
-    const int n_skip = (skip_flag != nullptr && __ldcg(skip_flag) != 0) ? skip : 0;
+    const bool skip = skip_flag != nullptr && __ldcg(skip_flag) != 0;
     const float *hp = p.partials + ((size_t)h * p.part_rows * rows) * PW;
     const size_t cta_stride = (size_t)rows * PW;
     const int items = rows * VPR;
@@ -283,21 +309,21 @@ __device__ __forceinline__ void merge_splits(const AttnParams &p, int h, int spl
         if (mine) {
             const float *col = hp + (size_t)(e / VPR) * PW + 4 * (e % VPR);
             const float *ml = hp + (size_t)(e / VPR) * PW + D;
-            for (int s0 = g; s0 < splits; s0 += groups * kMergeBatch) {
-                float4 v[kMergeBatch];
-                float2 w[kMergeBatch];
+            for (int s0 = lo + g; s0 < hi; s0 += groups * BATCH) {
+                float4 v[BATCH];
+                float2 w[BATCH];
 #pragma unroll
-                for (int i = 0; i < kMergeBatch; ++i) {
-                    const int s = min(s0 + i * groups, splits - 1);
+                for (int i = 0; i < BATCH; ++i) {
+                    const int s = min(s0 + i * groups, hi - 1);
                     v[i] = __ldcg(reinterpret_cast<const float4 *>(col + (size_t)s * cta_stride));
                     w[i] = __ldcg(reinterpret_cast<const float2 *>(ml + (size_t)s * cta_stride));
                 }
                 // the batch's own maximum first, so that its exponentials do not wait for one another
                 float mb = x.m;
 #pragma unroll
-                for (int i = 0; i < kMergeBatch; ++i) {
+                for (int i = 0; i < BATCH; ++i) {
                     const int s = s0 + i * groups;
-                    if (s >= splits || s < n_skip) w[i].x = -INFINITY;
+                    if (s >= hi || (skip && (s < p.splits1 || s == p.ticket_target))) w[i].x = -INFINITY;
                     mb = fmaxf(mb, w[i].x);
                 }
                 const float ms = (mb == -INFINITY) ? 0.f : mb;
@@ -306,7 +332,7 @@ __device__ __forceinline__ void merge_splits(const AttnParams &p, int h, int spl
                 x.l *= wx;
                 x.a.x *= wx; x.a.y *= wx; x.a.z *= wx; x.a.w *= wx;
 #pragma unroll
-                for (int i = 0; i < kMergeBatch; ++i) {
+                for (int i = 0; i < BATCH; ++i) {
                     if (w[i].x == -INFINITY) continue;   // (a CTA without units: its rows are zeros)
                     const float wv = fast_exp2(w[i].x - ms);
                     x.l = fmaf(w[i].y, wv, x.l);
@@ -330,7 +356,11 @@ __device__ __forceinline__ void merge_splits(const AttnParams &p, int h, int spl
                 }
             }
         }
-        if (mine && g == 0) {
+        if (mine && g == 0 && merged != nullptr) {
+            const int r = e / VPR, c4 = e % VPR;
+            *reinterpret_cast<float4 *>(merged + (size_t)r * PW + 4 * c4) = x.a;
+            if (c4 == 0) *reinterpret_cast<float2 *>(merged + (size_t)r * PW + D) = make_float2(x.m, x.l);
+        } else if (mine && g == 0) {
             const int r = e / VPR, c4 = e % VPR;
             const float inv = x.l > 0.f ? 1.f / x.l : 0.f;
             // row r = (query token, head of the group)
@@ -365,6 +395,14 @@ __device__ __forceinline__ void merge_splits(const AttnParams &p, int h, int spl
             }
         }
     }
+}
+
+template <typename T, int D, int THREADS>
+__device__ __forceinline__ void merge_partials(const AttnParams &p, int h, int lo, int hi, int rows,
+                                               const int32_t *skip_flag, float *merged, unsigned char *smem) {
+    const int groups = max(THREADS / (rows * (D / 4)), 1);
+    if (hi - lo <= kMergeBatchFew * groups) merge_range<T, D, THREADS, kMergeBatchFew>(p, h, lo, hi, rows, skip_flag, merged, smem);
+    else merge_range<T, D, THREADS, kMergeBatch>(p, h, lo, hi, rows, skip_flag, merged, smem);
 }
 
 // 16-bit element types: tensor-core kernel (attn_mma.cu).

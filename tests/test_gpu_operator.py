@@ -705,3 +705,30 @@ def test_one_library_call_equals_stage_by_stage(da, layout, counts):
     assert torch.equal(ms[0].cache_k, ms[1].cache_k)
     for m in ms:
         m.check_status()
+
+
+@pytest.mark.parametrize("ctas1,ctas2", [(1, 1), (2, 5), (3, 1), (18, 6), (55, 7), (148, 148)])
+@pytest.mark.parametrize("rep,dtype", [(1, torch.bfloat16), (8, torch.float16), (4, torch.bfloat16)])
+def test_two_launch_merge_at_any_number_of_partials(da, ctas1, ctas2, rep, dtype):
+    """The last CTA merges the partials of both launches; phase 1's own last one merges phase 1's into one before
+    that when phase 2 is still at work.  Few and many partials, steady steps and re-drawn queries (whose heads phase 2
+    redoes, phase 1 left out), against the single-launch layout; the ticket words are zero between steps."""
+    w = llama_layer_workload(seed=5, steps=12, dram_tokens=8192, n_kv_heads=2, rep=rep, lru=2048, local=256,
+                             top_k=128, needles=2, redraw_every=4, dtype=dtype)
+    a = da.DRAMAttention(device=DEV, dtype=dtype, **w.ctor_kwargs())
+    b = da.DRAMAttention(device=DEV, dtype=dtype, **w.ctor_kwargs())
+    a.phase1_ctas, a.phase2_ctas, b.overlap = ctas1, ctas2, False
+    for m in (a, b):
+        m.init_cache(w.k.to(DEV), w.v.to(DEV))
+    S = w.k.shape[1]
+    for i in range(12):
+        x = [t[i].to(DEV) for t in (w.xq, w.xk, w.xv)]
+        oa, ob = (m(*x, start_pos=S + i, stage="generate") for m in (a, b))
+        torch.cuda.synchronize()
+        assert_out_close(oa[0, 0].float().cpu(), ob[0, 0].float().cpu(), dtype, i)
+        assert torch.equal(a.lru_cache.hbm_kv_cache, b.lru_cache.hbm_kv_cache)
+        for buf, _, _ in a._ws.values():
+            assert not bool(buf[:1024].any())
+    assert a._can_overlap and a._overlap_supported(rep, dtype)
+    for m in (a, b):
+        m.check_status()
