@@ -311,9 +311,12 @@ static int run_attention(const AttnCall &c) {
     int splits0 = attn_splits(c.n_kv_heads);
     const int unit_splits = (c.n_prefix_tokens + c.local_capacity) / (2 * kUnitTokens * kAttnWarps) + 1;
     if (splits0 > unit_splits) splits0 = unit_splits;
-    const int part_rows = c.phase == 0 ? splits0 : c.splits1 + c.splits2 + 1;   // (the last: phase 1's merged into one)
-    if (c.workspace_bytes < (size_t)kCounterBytes + partial_bytes(c.n_kv_heads, part_rows, rows_max, c.head_dim))
+    const int ctas = c.phase == 0 ? splits0 : c.splits1 + c.splits2;
+    if (c.workspace_bytes < (size_t)kCounterBytes + partial_bytes(c.n_kv_heads, ctas, rows_max, c.head_dim))
         return DA_ERR_WORKSPACE;
+    // phase 1's partials merged into one, where the workspace (the same one for both launches) has room for one more
+    const size_t one_more = (size_t)kCounterBytes + partial_bytes(c.n_kv_heads, ctas + 1, rows_max, c.head_dim);
+    const int part_rows = ctas + (c.phase != 0 && c.workspace_bytes >= one_more ? 1 : 0);
 
     AttnParams p{};
     for (int g = 0; g < kAttnMaxPeers; ++g) p.peer_buf[g] = static_cast<uint2 *>(push.bufs[g]);
@@ -361,7 +364,7 @@ static int run_attention(const AttnCall &c) {
     p.s_total = c.n_q_tokens;
     p.part_rows = part_rows;
     p.part_offset = 0;
-    p.ticket_target = c.phase == 0 ? part_rows : part_rows - 1;
+    p.ticket_target = ctas;
     p.splits1 = 0;
     int splits = splits0;
     if (c.phase != 0) {
@@ -510,8 +513,8 @@ extern "C" int da_decode_attention_phase1_ctas(int n_kv_heads) {
 
 extern "C" size_t da_decode_attention_phased_workspace_bytes(int n_kv_heads, int rep, int head_dim) {
     if (n_kv_heads < 1 || rep < 1 || head_dim < 1) return 0;
-    // room for any choice of CTAs per head in the two launches, and for phase 1's partials merged into one
-    return (size_t)da::kCounterBytes + da::partial_bytes(n_kv_heads, 2 * da::kAttnMaxSplits + 1, rep, head_dim);
+    // room for any choice of CTAs per head in the two launches
+    return (size_t)da::kCounterBytes + da::partial_bytes(n_kv_heads, 2 * da::kAttnMaxSplits, rep, head_dim);
 }
 
 extern "C" int da_decode_attention_phased(int phase, const int32_t *order, const int32_t *n_evictable,

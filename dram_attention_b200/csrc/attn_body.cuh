@@ -293,7 +293,7 @@ __device__ __forceinline__ void decode_attention_body(const AttnParams &p, unsig
         const int done1 = (int)(old & (kTicketPhase2 - 1)), done2 = (int)((old & (kTicketMerged - 1)) / kTicketPhase2);
         int todo = kMergeNothing;
         if (done1 + done2 == p.ticket_target - 1) todo = (old & kTicketMerged) ? kMergeRest : kMergeAll;
-        else if (p.phase == 1 && done1 == p.splits1 - 1 && p.splits1 > 2) todo = kMergePhase1;
+        else if (p.phase == 1 && done1 == p.splits1 - 1 && p.splits1 > 2 && p.part_rows > p.ticket_target) todo = kMergePhase1;
         sh_merge = todo;
     }
     __syncthreads();

@@ -99,7 +99,7 @@ struct AttnParams {
     const int32_t *n_evictable;      // [2][n_kv_heads]
     int32_t *flip;                   // [n_kv_heads]
     const int32_t *redo;             // [n_kv_heads]
-    int part_rows;                   // partials per head in the workspace (two launches: one more than CTAs)
+    int part_rows;                   // partials per head in the workspace (two launches: one more than CTAs, if it has room)
     int part_offset;                 // first row this launch writes
     int ticket_target;               // CTAs of a head that take a ticket before the merge
     int splits1;                     // rows of phase 1 (first in the workspace)
