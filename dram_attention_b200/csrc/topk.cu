@@ -12,6 +12,29 @@ constexpr int kTopkThreads = 1024;
 constexpr int kTopkWarps = kTopkThreads / 32;
 constexpr int kTopkMaxK = 4096;
 
+// Where the selected pages go: the per-KV-head page list, or 64-bit ids of one row of the launch after the other.
+struct PageOut {
+    int32_t *list;
+    long long *ids;
+};
+struct PageDst {
+    int32_t *list;
+    long long *ids;
+    __device__ __forceinline__ void store(int i, uint32_t page) const {
+        if (ids) ids[i] = (long long)page;
+        else list[i] = (int32_t)page;
+    }
+};
+// Row `row` of the launch is ((token * n_kv_heads + hk) * rep + r).
+__device__ __forceinline__ PageDst row_destination(PageOut out, int row, int rows, int n_kv_heads, int rep, int k) {
+    if (out.ids) return {nullptr, out.ids + (size_t)row * k};
+    const int r = row % rep;
+    const int hk = (row / rep) % n_kv_heads;
+    const int tok = row / (rep * n_kv_heads);
+    const int n_tokens = rows / (n_kv_heads * rep);
+    return {out.list + (size_t)hk * n_tokens * rep * k + (size_t)(tok * rep + r) * k, nullptr};
+}
+
 // Candidates the ranking step can take: k plus half as many again (the selection stops
 // refining its threshold as soon as the keys above it and its whole bucket fit).
 __host__ __device__ inline int topk_candidate_capacity(int k) { return k + (k >> 1); }
@@ -121,7 +144,7 @@ __device__ __forceinline__ void descending_crossing(const int *hist, int need, i
 // composite keys; the first k leave.  The candidate array is read two entries per 128-bit load; with
 // m odd the pad entry is the largest possible key and counts for nobody.  `rank` is scratch of m ints.
 __device__ __forceinline__ void rank_candidates(unsigned long long *cand, int *rank, int m, int k,
-                                                int32_t *__restrict__ dst, int tid) {
+                                                PageDst dst, int tid) {
     for (int e = tid; e < m; e += kTopkThreads) rank[e] = 0;
     if (tid == 0 && (m & 1)) cand[m] = ~0ull;
     __syncthreads();
@@ -153,14 +176,14 @@ __device__ __forceinline__ void rank_candidates(unsigned long long *cand, int *r
     __syncthreads();
     for (int e = tid; e < m; e += kTopkThreads) {
         const int rk = rank[e];
-        if (rk < k) dst[rk] = (int32_t)(cand[e] & 0xffffffffu);
+        if (rk < k) dst.store(rk, (uint32_t)cand[e]);
     }
 }
 
 // One row, one CTA: the whole selection.  `dst` receives the k page ids in (score descending,
 // page id ascending) order.
 template <int IPT>
-__device__ __forceinline__ void topk_row(const float *__restrict__ srow, int n_pages, int k, int32_t *__restrict__ dst,
+__device__ __forceinline__ void topk_row(const float *__restrict__ srow, int n_pages, int k, PageDst dst,
                                          unsigned char *smem_raw) {
     const int cap = topk_candidate_capacity(k);
     unsigned long long *cand = reinterpret_cast<unsigned long long *>(smem_raw);  // [cap + 2]
@@ -331,7 +354,7 @@ __device__ __forceinline__ void topk_row(const float *__restrict__ srow, int n_p
             const int last = first + count_of[b];
             int c = first;
             for (int j = first; j < last; ++j) c += cand[j] < v;
-            if (c < k) dst[c] = (int32_t)(v & 0xffffffffu);
+            if (c < k) dst.store(c, (uint32_t)v);
         }
         return;
     }
@@ -409,18 +432,9 @@ __device__ __forceinline__ void topk_row(const float *__restrict__ srow, int n_p
     rank_candidates(cand, rank, m, k, dst, tid);
 }
 
-// Where row `row` of the launch ((token * n_kv_heads + hk) * rep + r) goes in the per-KV-head page list.
-__device__ __forceinline__ int32_t *row_destination(int32_t *page_list, int row, int rows, int n_kv_heads, int rep, int k) {
-    const int r = row % rep;
-    const int hk = (row / rep) % n_kv_heads;
-    const int tok = row / (rep * n_kv_heads);
-    const int n_tokens = rows / (n_kv_heads * rep);
-    return page_list + (size_t)hk * n_tokens * rep * k + (size_t)(tok * rep + r) * k;
-}
-
 template <int IPT>
 __global__ void __launch_bounds__(kTopkThreads)
-topk_pages_kernel(const float *__restrict__ scores, int32_t *__restrict__ page_list, int n_kv_heads, int rep,
+topk_pages_kernel(const float *__restrict__ scores, PageOut page_list, int n_kv_heads, int rep,
                   int n_pages, int k) {
     if (threadIdx.x == 0) trace_stamp(1, blockIdx.x, 0);
     // on whichever path the kernel leaves: thread 0's end stamp
@@ -481,12 +495,12 @@ __device__ __forceinline__ void dsmem_st_u64(uint32_t addr, unsigned long long v
 // The fall-back of the cluster kernel, kept out of line so that the common path stays small in the
 // instruction cache.
 __device__ __noinline__ void topk_row_fallback(const float *__restrict__ srow, int n_pages, int k,
-                                               int32_t *__restrict__ dst, unsigned char *smem_raw) {
+                                               PageDst dst, unsigned char *smem_raw) {
     topk_row<0>(srow, n_pages, k, dst, smem_raw);
 }
 
 __global__ void __launch_bounds__(kTopkThreads)
-topk_pages_cluster_kernel(const float *__restrict__ scores, int32_t *__restrict__ page_list, int n_kv_heads, int rep,
+topk_pages_cluster_kernel(const float *__restrict__ scores, PageOut page_list, int n_kv_heads, int rep,
                           int n_pages, int k) {
     if (threadIdx.x == 0) trace_stamp(1, blockIdx.x, 0);
     struct EndStamp {
@@ -512,7 +526,7 @@ topk_pages_cluster_kernel(const float *__restrict__ scores, int32_t *__restrict_
     const int row = blockIdx.x / kTopkCluster;
     const int rows = gridDim.x / kTopkCluster;
     const float *srow = scores + (size_t)row * n_pages;
-    int32_t *dst = row_destination(page_list, row, rows, n_kv_heads, rep, k);
+    const PageDst dst = row_destination(page_list, row, rows, n_kv_heads, rep, k);
     // this CTA's part of the row: `per` pages from `base` (a multiple of 4 pages, so that every part starts aligned)
     const int per = (((n_pages + kTopkCluster - 1) / kTopkCluster) + 3) & ~3;
     const int base = min((int)crank * per, n_pages);
@@ -647,7 +661,7 @@ topk_pages_cluster_kernel(const float *__restrict__ scores, int32_t *__restrict_
             const int last = first + total[b];
             int c = first;
             for (int j = first; j < last; ++j) c += cand[j] < v;
-            if (c < k) dst[c] = (int32_t)(v & 0xffffffffu);
+            if (c < k) dst.store(c, (uint32_t)v);
         }
         return;
     }
@@ -681,7 +695,7 @@ template <bool VEC> __device__ __forceinline__ int group_element(int it, int q, 
 
 template <int PER, bool VEC>
 __global__ void __launch_bounds__(kTopkThreads)
-topk_pages_groups_kernel(const float *__restrict__ scores, int32_t *__restrict__ page_list, int n_kv_heads, int rep,
+topk_pages_groups_kernel(const float *__restrict__ scores, PageOut page_list, int n_kv_heads, int rep,
                          int n_pages, int k) {
     if (threadIdx.x == 0) trace_stamp(1, blockIdx.x, 0);
     struct EndStamp {
@@ -705,7 +719,7 @@ topk_pages_groups_kernel(const float *__restrict__ scores, int32_t *__restrict__
     const int warp = tid >> 5;
     const int row = blockIdx.x;
     const float *srow = scores + (size_t)row * n_pages;
-    int32_t *dst = row_destination(page_list, row, gridDim.x, n_kv_heads, rep, k);
+    const PageDst dst = row_destination(page_list, row, gridDim.x, n_kv_heads, rep, k);
 
     if (tid < 256) {
         hist[0][tid] = 0;
@@ -874,12 +888,12 @@ topk_pages_groups_kernel(const float *__restrict__ scores, int32_t *__restrict__
         const int last = first + count_of[b];
         int c = first;
         for (int j = first; j < last; ++j) c += cand[j] < v;
-        if (c < k) dst[c] = (int32_t)(v & 0xffffffffu);
+        if (c < k) dst.store(c, (uint32_t)v);
     }
 }
 
 template <int IPT>
-static cudaError_t launch_topk(const float *scores, int32_t *page_list, int rows, int n_kv_heads, int rep,
+static cudaError_t launch_topk(const float *scores, PageOut page_list, int rows, int n_kv_heads, int rep,
                                int n_pages, int k, cudaStream_t stream) {
     // opt in to > 48 KB of dynamic shared memory once per device
     static bool attr_set[64] = {};
@@ -902,7 +916,7 @@ static cudaError_t launch_topk(const float *scores, int32_t *page_list, int rows
 }
 
 template <int PER, bool VEC>
-static cudaError_t launch_topk_groups(const float *scores, int32_t *page_list, int rows, int n_kv_heads, int rep,
+static cudaError_t launch_topk_groups(const float *scores, PageOut page_list, int rows, int n_kv_heads, int rep,
                                       int n_pages, int k, cudaStream_t stream) {
     const int cap = topk_candidate_capacity(k);      // at most 2048 here: 24 KB, no opt-in needed
     const size_t smem = (size_t)(cap + 2) * sizeof(unsigned long long) + (size_t)cap * sizeof(int);
@@ -912,14 +926,14 @@ static cudaError_t launch_topk_groups(const float *scores, int32_t *page_list, i
 }
 
 template <int PER>
-static cudaError_t launch_topk_groups(const float *scores, int32_t *page_list, int rows, int n_kv_heads, int rep,
+static cudaError_t launch_topk_groups(const float *scores, PageOut page_list, int rows, int n_kv_heads, int rep,
                                       int n_pages, int k, cudaStream_t stream) {
     if (n_pages % 4 == 0 && ((uintptr_t)scores & 15) == 0)
         return launch_topk_groups<PER, true>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, stream);
     return launch_topk_groups<PER, false>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, stream);
 }
 
-static cudaError_t launch_topk_cluster(const float *scores, int32_t *page_list, int rows, int n_kv_heads, int rep,
+static cudaError_t launch_topk_cluster(const float *scores, PageOut page_list, int rows, int n_kv_heads, int rep,
                                        int n_pages, int k, cudaStream_t stream) {
     static bool attr_set[64] = {};
     int dev = 0;
@@ -954,9 +968,9 @@ static cudaError_t launch_topk_cluster(const float *scores, int32_t *page_list, 
 
 }  // namespace da
 
-extern "C" int da_topk_pages_wide(const float *scores, int32_t *page_list, int n_tokens, int n_kv_heads, int rep,
-                                  int n_pages, int k, int sm_budget, da_stream_t stream) {
-    if (!scores || !page_list) return DA_ERR_NULL;
+static int select_pages(const float *scores, da::PageOut page_list, int n_tokens, int n_kv_heads, int rep, int n_pages,
+                        int k, int sm_budget, da_stream_t stream) {
+    if (!scores || (!page_list.list && !page_list.ids)) return DA_ERR_NULL;
     if (n_tokens < 1 || n_kv_heads < 1 || rep < 1 || n_pages < 1 || k < 1 || k > n_pages || sm_budget < 0)
         return DA_ERR_SHAPE;
     if (k > da::kTopkMaxK) return DA_ERR_UNSUPPORTED;
@@ -979,6 +993,16 @@ extern "C" int da_topk_pages_wide(const float *scores, int32_t *page_list, int n
         e = da::launch_topk_cluster(scores, page_list, rows, n_kv_heads, rep, n_pages, k, s);
     else e = da::launch_topk<0>(scores, page_list, rows, n_kv_heads, rep, n_pages, k, s);
     return (int)e;
+}
+
+extern "C" int da_topk_pages_wide(const float *scores, int32_t *page_list, int n_tokens, int n_kv_heads, int rep,
+                                  int n_pages, int k, int sm_budget, da_stream_t stream) {
+    return select_pages(scores, da::PageOut{page_list, nullptr}, n_tokens, n_kv_heads, rep, n_pages, k, sm_budget, stream);
+}
+
+extern "C" int da_topk_page_ids(const float *scores, long long *page_ids, int n_tokens, int n_kv_heads, int rep,
+                                int n_pages, int k, da_stream_t stream) {
+    return select_pages(scores, da::PageOut{nullptr, page_ids}, n_tokens, n_kv_heads, rep, n_pages, k, 0, stream);
 }
 
 extern "C" int da_topk_pages(const float *scores, int32_t *page_list, int n_tokens, int n_kv_heads, int rep,

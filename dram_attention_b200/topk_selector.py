@@ -97,8 +97,12 @@ class IPUpperboundTopKSelector:
         """Top-k page ids for each token and query head: int64 (S, Hk, rep, k), as
         the reference's top_k (dram_attention/topk_selector.py:37-61)."""
         bsz, seq_len, num_q_heads, _ = q.shape
+        k = min(k, self.num_pages)
         with torch.cuda.device(q.device):
-            _, page_list = self.page_list_(q, k)
-        rep = num_q_heads // self.num_kv_heads
-        kk = page_list.shape[1] // (seq_len * rep)
-        return page_list.view(self.num_kv_heads, seq_len, rep, kk).swapaxes(0, 1).to(torch.int64)
+            scores = self.score_(q, k)
+            rep = num_q_heads // self.num_kv_heads
+            ids = torch.empty(seq_len, self.num_kv_heads, rep, k, dtype=torch.int64, device=scores.device)
+            _native.check(_native.lib().da_topk_page_ids(
+                scores.data_ptr(), ids.data_ptr(), seq_len, self.num_kv_heads, rep, self.num_pages, k,
+                _native.stream_ptr()), "da_topk_page_ids")
+        return ids

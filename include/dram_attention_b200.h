@@ -138,6 +138,14 @@ DA_API int da_topk_pages_wide(const float *scores, int32_t *page_list,
                        int sm_budget, da_stream_t stream);
 
 /*
+ * The same selection as 64-bit ids: page_ids (n_tokens, n_kv_heads, rep, k) int64, the result of the reference's top_k
+ * (dram_attention/topk_selector.py:37-61), written by the selection itself.
+ */
+DA_API int da_topk_page_ids(const float *scores, long long *page_ids,
+                     int n_tokens, int n_kv_heads, int rep, int n_pages, int k,
+                     da_stream_t stream);
+
+/*
  * LRU slot-table update, one call for all KV heads.  Replaces load_lru_cache_()
  * without its payload copy: _update_page_access_time_
  * (dram_attention/lru_triton_kernel.py:110-137), the stable argsort of the

@@ -811,3 +811,16 @@ def test_topk_long_rows_by_group_maxima(da, pages, k, kind):
                                                    _native.stream_ptr()))
     want = torch.sort(sc, dim=-1, descending=True, stable=True).indices[:, :k].reshape(1, -1).to(torch.int32)
     assert torch.equal(out.cpu(), want)
+
+
+@pytest.mark.parametrize("pages,k,s", [(100, 8, 3), (5000, 300, 2), (12000, 64, 1), (40000, 200, 2), (65536, 1500, 1)])
+def test_page_ids_are_the_page_list(da, pages, k, s):
+    """The 64-bit ids of every selection kernel, several tokens included, against the page list of the same scores."""
+    from dram_attention_b200 import _native
+    hk, rep = 2, 2
+    sc = torch.randn(s, hk * rep, pages, generator=_g(pages)).to(DEV)
+    ids = torch.full((s, hk, rep, k), -1, dtype=torch.int64, device=DEV)
+    _native.check(_native.lib().da_topk_page_ids(sc.data_ptr(), ids.data_ptr(), s, hk, rep, pages, k,
+                                                 _native.stream_ptr()))
+    lst = _topk(da, sc.cpu(), hk, rep, k)
+    assert torch.equal(ids.cpu(), lst.view(hk, s, rep, k).swapaxes(0, 1).to(torch.int64))
