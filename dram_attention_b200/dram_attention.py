@@ -96,11 +96,22 @@ class DRAMAttention(torch.nn.Module):
         dram_kv_cache_size = (seqlen - self.local_cache_size + self.page_size) // self.page_size * self.page_size
         dram_k_cache = k_cache[:, :dram_kv_cache_size]
         dram_v_cache = v_cache[:, :dram_kv_cache_size]
+
+        def fill_window():
+            length = seqlen - dram_kv_cache_size
+            self.cache_k[:, :length].copy_(k_cache[:, dram_kv_cache_size:], non_blocking=True)
+            self.cache_v[:, :length].copy_(v_cache[:, dram_kv_cache_size:], non_blocking=True)
+
+        def beside_construction():
+            beside()
+            fill_window()
+
         if dram_kv_cache_size > self.lru_hbm_cache_size:
             lru_cache = LRUCache(
                 k_cache=dram_k_cache[0].transpose(0, 1), v_cache=dram_v_cache[0].transpose(0, 1),
                 page_size=self.page_size, top_k=self.top_k // self.page_size,
-                lru_hbm_cache_size=self.lru_hbm_cache_size, device=self.device, _beside=beside)
+                lru_hbm_cache_size=self.lru_hbm_cache_size, device=self.device,
+                _beside=None if beside is None else beside_construction)
             # the kernel that fetches on the fly needs its 16-token units inside one page
             self._can_fuse = self.page_size % 16 == 0
             self._can_overlap = self._can_fuse   # refined per GQA group size at the first generate call
@@ -115,9 +126,8 @@ class DRAMAttention(torch.nn.Module):
             self._can_overlap = False
         self.lru_cache = lru_cache
         self.dram_kv_cache_size = dram_kv_cache_size
-        L = seqlen - dram_kv_cache_size
-        self.cache_k[:, :L].copy_(k_cache[:, dram_kv_cache_size:], non_blocking=True)
-        self.cache_v[:, :L].copy_(v_cache[:, dram_kv_cache_size:], non_blocking=True)
+        if beside is None or isinstance(lru_cache, DummyCache):
+            fill_window()
 
     def init_cache_sharing(self, other: "DRAMAttention") -> None:
         """Initialise this operator as `init_cache` would with the prefill KV `other` was given,
