@@ -48,7 +48,8 @@ __device__ __forceinline__ void decode_attention_body(const AttnParams &p, unsig
     constexpr int PW = PartialRow<D>::kWidth;
     constexpr int THREADS = WARPS * 32;
     constexpr float NEG_INF = -INFINITY;
-    static_assert(STAGES * STAGEB >= kAttnMaxRows * PW * (int)sizeof(float), "a warp's ring holds its partial");
+    static_assert(STAGES * STAGEB >= (E == 2 ? kAttnWideRows : kAttnMaxRows) * PW * (int)sizeof(float),
+                  "a warp's ring holds its partial");
 
     __shared__ __align__(8) uint64_t bars[WARPS][STAGES];
     __shared__ __align__(16) uint4 plan_tab[WARPS][kRoundUnits];

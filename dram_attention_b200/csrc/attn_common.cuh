@@ -12,7 +12,8 @@ constexpr int kUnitTokens = 16;
 constexpr int kCounterBytes = 1024;
 constexpr int kAttnSms = 148;
 constexpr int kAttnMaxSplits = 148;
-constexpr int kAttnMaxRows = 16;       // query rows (tokens x GQA group) of one KV head per launch
+constexpr int kAttnMaxRows = 16;       // query rows (tokens x GQA group) of one KV head that the workspaces are sized for
+constexpr int kAttnWideRows = 32;      // ... and the most that a launch takes (16-bit types)
 constexpr int kRoundUnits = 32;        // units a warp plans at a time (one per lane)
 
 // CTAs per head ("splits").  Every CTA of every launch fills an SM on its own (12 warps, nearly all of the shared

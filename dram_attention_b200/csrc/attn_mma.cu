@@ -241,6 +241,160 @@ struct MmaMath {
     }
 };
 
+// Up to 32 query rows (several query tokens per call) in one pass over the keys and values, as two m16 tiles that share
+// every B fragment.  Their accumulators take 128 registers per thread, so a CTA has 8 warps of up to 255, with three
+// stages each (the bytes in flight of 12 x 2), and the Q fragments come from shared memory instead of registers.
+template <typename T, int D_>
+struct MmaMathWide {
+    using Elem = T;
+    static constexpr int kD = D_;
+    static constexpr int ROWB = kD * 2;
+    static constexpr int kPitch = 2 * ROWB + 16;
+    static constexpr int STAGEB = kUnitTokens * kPitch;
+    static constexpr bool kPerTokenCopy = true;
+    static constexpr int KSTEPS = kD / 16;
+    static constexpr int NT = kD / 8;
+    static constexpr int kRows = 32;
+    static constexpr int QP = ROWB + 16;                  // pitch of a query row in shared memory
+
+    struct State {
+        const unsigned char *q;       // this lane's row address of the first A fragment
+        float m_run[2][2], l_part[2][2];
+        float o[2][NT][4];
+        int back[2][2];
+    };
+
+    __device__ __forceinline__ static void init(State &st, const AttnParams &p, int h, int lane, int rows) {
+        __shared__ __align__(16) unsigned char q_sh[kRows * QP];
+        const int hq = p.n_kv_heads * p.rep;
+        for (int i = threadIdx.x; i < kRows * (ROWB / 16); i += blockDim.x) {
+            const int r = i / (ROWB / 16), c = i % (ROWB / 16);
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (r < rows)
+                v = *reinterpret_cast<const uint4 *>(
+                    p.q + ((size_t)(p.q_tok0 + r / p.rep) * hq + (size_t)h * p.rep + r % p.rep) * ROWB + 16 * c);
+            *reinterpret_cast<uint4 *>(q_sh + r * QP + 16 * c) = v;
+        }
+        __syncthreads();
+        st.q = q_sh + (((lane >> 3) & 1) * 8 + (lane & 7)) * QP + (lane >> 4) * 16;
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int r = 16 * mt + 8 * half + (lane >> 2);
+                st.back[mt][half] = r < rows ? p.s_total - 1 - (p.q_tok0 + r / p.rep) : 0;
+                st.m_run[mt][half] = -INFINITY;
+                st.l_part[mt][half] = 0.f;
+            }
+#pragma unroll
+            for (int d = 0; d < NT; ++d) st.o[mt][d][0] = st.o[mt][d][1] = st.o[mt][d][2] = st.o[mt][d][3] = 0.f;
+        }
+    }
+
+    __device__ __forceinline__ static void consume(State &st, const unsigned char *sb, int avail, int lane,
+                                                   float scale_log2) {
+        constexpr float NEG_INF = -INFINITY;
+        const int qd = lane & 3;
+        const int lm = lane >> 3, lr = lane & 7;
+        const int k_off = lr * kPitch + lm * 16;
+        const int v_off = ROWB + ((lm & 1) * 8 + lr) * kPitch + (lm >> 1) * 16;
+
+        // ---- S = Q K^T: two m-tiles by two n-tiles of 8 tokens ----------------------------
+        float s[2][2][4] = {};
+#pragma unroll
+        for (int kp = 0; kp < KSTEPS / 2; ++kp) {
+            uint32_t b[4], c[4];
+            ldmatrix_x4(b, sb + k_off + kp * 64);                 // tokens 0..7, channels 32kp .. 32kp+31
+            ldmatrix_x4(c, sb + k_off + 8 * kPitch + kp * 64);    // tokens 8..15
+#pragma unroll
+            for (int k2 = 0; k2 < 2; ++k2) {
+#pragma unroll
+                for (int mt = 0; mt < 2; ++mt) {
+                    uint32_t a[4];
+                    ldmatrix_x4(a, st.q + mt * 16 * QP + (2 * kp + k2) * 32);
+                    MmaTraits<T>::mma16(s[mt][0], a[0], a[1], a[2], a[3], b[2 * k2], b[2 * k2 + 1]);
+                    MmaTraits<T>::mma16(s[mt][1], a[0], a[1], a[2], a[3], c[2 * k2], c[2 * k2 + 1]);
+                }
+            }
+        }
+        uint32_t pa[2][2][2];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                // this lane: row lane/4 + 8*half + 16*mt, tokens 2qd, 2qd+1, 8+2qd, 9+2qd
+                const int lim = avail - st.back[mt][half];
+                float v0 = s[mt][0][2 * half] * scale_log2, v1 = s[mt][0][2 * half + 1] * scale_log2;
+                float v2 = s[mt][1][2 * half] * scale_log2, v3 = s[mt][1][2 * half + 1] * scale_log2;
+                if (2 * qd >= lim) v0 = NEG_INF;
+                if (2 * qd + 1 >= lim) v1 = NEG_INF;
+                if (8 + 2 * qd >= lim) v2 = NEG_INF;
+                if (9 + 2 * qd >= lim) v3 = NEG_INF;
+                float mx = fmaxf(fmaxf(v0, v1), fmaxf(v2, v3));
+                mx = fmaxf(mx, __shfl_xor_sync(DA_FULL_MASK, mx, 1));
+                mx = fmaxf(mx, __shfl_xor_sync(DA_FULL_MASK, mx, 2));
+                const float mnew = fmaxf(st.m_run[mt][half], mx);
+                const float msafe = (mnew == NEG_INF) ? 0.f : mnew;
+                const float alpha = fast_exp2(st.m_run[mt][half] - msafe);
+                v0 = fast_exp2(v0 - msafe);
+                v1 = fast_exp2(v1 - msafe);
+                v2 = fast_exp2(v2 - msafe);
+                v3 = fast_exp2(v3 - msafe);
+                st.l_part[mt][half] = st.l_part[mt][half] * alpha + ((v0 + v1) + (v2 + v3));
+                st.m_run[mt][half] = mnew;
+                if (__any_sync(DA_FULL_MASK, alpha != 1.f)) {
+#pragma unroll
+                    for (int d = 0; d < NT; ++d) {
+                        st.o[mt][d][2 * half] *= alpha;
+                        st.o[mt][d][2 * half + 1] *= alpha;
+                    }
+                }
+                pa[mt][half][0] = MmaTraits<T>::pack(v0, v1);
+                pa[mt][half][1] = MmaTraits<T>::pack(v2, v3);
+            }
+        }
+
+        // ---- O += P V ---------------------------------------------------------------------
+#pragma unroll
+        for (int dp = 0; dp < NT / 2; ++dp) {
+            uint32_t b[4];
+            ldmatrix_x4_trans(b, sb + v_off + dp * 32);           // channels 16dp .. 16dp+15, all 16 tokens
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) {
+                MmaTraits<T>::mma16(st.o[mt][2 * dp], pa[mt][0][0], pa[mt][1][0], pa[mt][0][1], pa[mt][1][1], b[0], b[1]);
+                MmaTraits<T>::mma16(st.o[mt][2 * dp + 1], pa[mt][0][0], pa[mt][1][0], pa[mt][0][1], pa[mt][1][1], b[2], b[3]);
+            }
+        }
+    }
+
+    __device__ __forceinline__ static void publish(State &st, float *red, int lane, int rows) {
+        constexpr int PW = PartialRow<kD>::kWidth;
+        const int qd = lane & 3;
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                float l = st.l_part[mt][half];
+                l += __shfl_xor_sync(DA_FULL_MASK, l, 1);
+                l += __shfl_xor_sync(DA_FULL_MASK, l, 2);
+                const int r = 16 * mt + 8 * half + (lane >> 2);
+                if (r < rows) {
+#pragma unroll
+                    for (int d = 0; d < NT; ++d) {
+                        red[r * PW + 8 * d + 2 * qd] = st.o[mt][d][2 * half];
+                        red[r * PW + 8 * d + 2 * qd + 1] = st.o[mt][d][2 * half + 1];
+                    }
+                    if (qd == 0) {
+                        red[r * PW + kD] = st.m_run[mt][half];
+                        red[r * PW + kD + 1] = l;
+                    }
+                }
+            }
+        }
+    }
+};
+
+constexpr int kMmaWideWarps = 8, kMmaWideStages = 3;
 constexpr int kMmaStages = 2;   // per warp: 12 x 2 stages are 203 KB of an SM's shared memory for head_dim 128
 
 template <typename T, int D, bool FULL>
@@ -249,11 +403,14 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 1) decode_attention_mma_kerne
     decode_attention_body<MmaMath<T, D, FULL>, kAttnWarps, kMmaStages>(p, smem);
 }
 
-template <typename T, int D, bool FULL>
+template <typename T, int D>
+__global__ void __launch_bounds__(kMmaWideWarps * 32, 1) decode_attention_mma_wide_kernel(const AttnParams p) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    decode_attention_body<MmaMathWide<T, D>, kMmaWideWarps, kMmaWideStages>(p, smem);
+}
+
+template <typename T, int D, int WARPS, int SMEM, void (*kern)(const AttnParams)>
 static cudaError_t launch_mma(const AttnParams &p, int n_kv_heads, int splits, cudaStream_t stream) {
-    using M = MmaMath<T, D, FULL>;
-    constexpr int SMEM = kAttnWarps * kMmaStages * M::STAGEB;
-    auto kern = decode_attention_mma_kernel<T, D, FULL>;
     static bool attr_set[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -267,15 +424,19 @@ static cudaError_t launch_mma(const AttnParams &p, int n_kv_heads, int splits, c
     dim3 grid(splits, n_kv_heads);
     // phase 1 runs on a stream of its own beside the kernels of the step; the other launches follow
     // the LRU update in their stream and may move onto the SMs while it is still running
-    if (p.phase != 1) return launch_dependent(kern, grid, dim3(kAttnWarps * 32), (size_t)SMEM, stream, p);
-    kern<<<grid, kAttnWarps * 32, SMEM, stream>>>(p);
+    if (p.phase != 1) return launch_dependent(kern, grid, dim3(WARPS * 32), (size_t)SMEM, stream, p);
+    kern<<<grid, WARPS * 32, SMEM, stream>>>(p);
     return cudaGetLastError();
 }
 
 template <typename T, int D>
 static cudaError_t launch_mma_d(const AttnParams &p, int n_kv_heads, int splits, cudaStream_t stream) {
-    if (p.n_q * p.rep > 8) return launch_mma<T, D, true>(p, n_kv_heads, splits, stream);
-    return launch_mma<T, D, false>(p, n_kv_heads, splits, stream);
+    constexpr int kStageBytes = MmaMath<T, D, false>::STAGEB;
+    constexpr int kSmem = kAttnWarps * kMmaStages * kStageBytes, kWideSmem = kMmaWideWarps * kMmaWideStages * kStageBytes;
+    const int rows = p.n_q * p.rep;
+    if (rows > 16) return launch_mma<T, D, kMmaWideWarps, kWideSmem, decode_attention_mma_wide_kernel<T, D>>(p, n_kv_heads, splits, stream);
+    if (rows > 8) return launch_mma<T, D, kAttnWarps, kSmem, decode_attention_mma_kernel<T, D, true>>(p, n_kv_heads, splits, stream);
+    return launch_mma<T, D, kAttnWarps, kSmem, decode_attention_mma_kernel<T, D, false>>(p, n_kv_heads, splits, stream);
 }
 
 template <typename T>

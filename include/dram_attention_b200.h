@@ -305,8 +305,8 @@ DA_API int da_decode_attention(const void *q,
  * q, out       (n_q_tokens, n_kv_heads * rep, head_dim); new_k, new_v (n_q_tokens, n_kv_heads,
  *              head_dim); lse_out optional (n_q_tokens, n_kv_heads * rep)
  * workspace    da_decode_attention_tokens_workspace_bytes() bytes
- * One launch covers 16 / rep tokens for 16-bit types (8 / rep for float32); longer calls are
- * several launches on `stream`.  Requires rep <= 16 (8 for float32), n_q_tokens <= local_capacity.
+ * One launch covers 16 / rep tokens for 16-bit types (8 / rep for float32), or 32 / rep of a longer call where the
+ * workspace has room for as many rows (two or more KV heads); longer calls are several launches on `stream`.  Requires rep <= 16 (8 for float32), n_q_tokens <= local_capacity.
  */
 DA_API size_t da_decode_attention_tokens_workspace_bytes(int n_kv_heads, int rep, int head_dim,
                         int n_q_tokens);

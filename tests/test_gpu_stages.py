@@ -824,3 +824,46 @@ def test_page_ids_are_the_page_list(da, pages, k, s):
                                                  _native.stream_ptr()))
     lst = _topk(da, sc.cpu(), hk, rep, k)
     assert torch.equal(ids.cpu(), lst.view(hk, s, rep, k).swapaxes(0, 1).to(torch.int64))
+
+
+# ------------------------------------------------------- attention of many query rows ----
+
+@pytest.mark.parametrize("tokens,hk,rep,d,dtype", [
+    (17, 2, 1, 128, torch.bfloat16), (5, 8, 4, 128, torch.bfloat16), (8, 2, 4, 64, torch.float16),
+    (9, 2, 4, 128, torch.float16),      # 32 rows, then 4
+    (6, 3, 8, 128, torch.bfloat16),     # 32 rows, then 16
+    (2, 4, 16, 64, torch.bfloat16),
+    (7, 1, 4, 128, torch.bfloat16),     # one KV head: no room in the workspace for 32 rows, two launches of 16
+])
+@pytest.mark.parametrize("prefix,window", [(1600, 700), (40, 64)])
+def test_attention_of_more_than_16_rows(da, tokens, hk, rep, d, dtype, prefix, window):
+    """Several query tokens per call with more than 16 query rows per KV head, against the oracle's two masked parts in
+    float64 (as the operator's own several-token test, with the suite's tolerance)."""
+    from dram_attention_b200 import _native
+    lib = _native.lib()
+    g = _g(tokens * 100 + prefix)
+    hq, dram, t0 = hk * rep, 4096, window - tokens - 3
+    kv = torch.randn(hk, prefix, 2, d, generator=g).to(dtype)
+    lk, lv = (torch.randn(window, hk, d, generator=g).to(dtype) for _ in range(2))
+    q = (2 * torch.randn(tokens, hq, d, generator=g)).to(dtype)
+    nk, nv = (torch.randn(tokens, hk, d, generator=g).to(dtype) for _ in range(2))
+    dq, dkv, dlk, dlv, dnk, dnv = (t.to(DEV) for t in (q, kv, lk, lv, nk, nv))
+    out = torch.full_like(dq, float("nan"))
+    lse = torch.empty(tokens, hq, dtype=torch.float32, device=DEV)
+    nbytes = lib.da_decode_attention_tokens_workspace_bytes(hk, rep, d, tokens)
+    ws = torch.zeros(nbytes, dtype=torch.uint8, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    for _ in range(2):      # the second call finds the workspace as the first left it
+        _native.check(lib.da_decode_attention_tokens(
+            dq.data_ptr(), tokens, dkv.data_ptr(), prefix * 2 * d, prefix, dlk.data_ptr(), dlv.data_ptr(), hk * d, d, window,
+            dnk.data_ptr(), dnv.data_ptr(), 0, dram + t0, dram, out.data_ptr(), lse.data_ptr(), ws.data_ptr(), nbytes,
+            status.data_ptr(), hk, rep, d, _native.dtype_code(dtype), _native.stream_ptr()))
+    torch.cuda.synchronize()
+    assert int(status) == 0 and not bool(ws[:1024].any())
+    lk[t0:t0 + tokens], lv[t0:t0 + tokens] = nk, nv
+    assert torch.equal(dlk.cpu(), lk) and torch.equal(dlv.cpu(), lv)
+    po, pl = orc.attend_tokens(q.float(), kv[:, :, 0].transpose(0, 1).float(), kv[:, :, 1].transpose(0, 1).float())
+    so, sl = orc.attend_tokens(q.float(), lk[:t0 + tokens].float(), lv[:t0 + tokens].float())
+    for j in range(tokens):
+        assert_out_close(out[j].float().cpu(), orc.combine(po[j], so[j], pl[j], sl[j]), dtype, j)
+        assert torch.allclose(lse[j].double().cpu(), torch.logaddexp(pl[j], sl[j]).double(), atol=2e-3)
