@@ -141,6 +141,11 @@ cudaError_t trace_set_gather(void *buffer);
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// The launches of that chain go ahead of work of the default priority when an SM falls free: the first attention launch
+// of another sequence on another stream takes whole SMs, as the selection does, and kept it waiting for 60 us.  Eight
+// sequences of 64K on four streams: 301 -> 291 us (with the scorer too: 296); a single sequence is unchanged.
+constexpr int kChainPriority = -1;
+
 template <typename... KArgs, typename... Args>
 static inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                            cudaStream_t stream, Args... args) {
@@ -149,11 +154,13 @@ static inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, 
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePriority;
+    attr[1].val.priority = kChainPriority;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
