@@ -147,8 +147,8 @@ __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("grid
 constexpr int kChainPriority = -1;
 
 template <typename... KArgs, typename... Args>
-static inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                           cudaStream_t stream, Args... args) {
+static inline cudaError_t launch_dependent_at(int priority, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                              cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -158,10 +158,16 @@ static inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributePriority;
-    attr[1].val.priority = kChainPriority;
+    attr[1].val.priority = priority;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = priority != 0 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                           cudaStream_t stream, Args... args) {
+    return launch_dependent_at(0, kernel, grid, block, smem, stream, args...);
 }
 
 // The scorer behind da_score_pages; `started` (may be null) is recorded when all its CTAs have begun.

@@ -909,7 +909,7 @@ static cudaError_t launch_topk(const float *scores, PageOut page_list, int rows,
     }
     const int cap = topk_candidate_capacity(k);
     const size_t smem = (size_t)(cap + 2) * sizeof(unsigned long long) + (size_t)cap * sizeof(int);
-    const cudaError_t le = launch_dependent(topk_pages_kernel<IPT>, dim3(rows), dim3(kTopkThreads), (size_t)smem, stream,
+    const cudaError_t le = launch_dependent_at(kChainPriority, topk_pages_kernel<IPT>, dim3(rows), dim3(kTopkThreads), (size_t)smem, stream,
                                             scores, page_list, n_kv_heads, rep, n_pages, k);
     if (le != cudaSuccess) return le;
     return cudaGetLastError();
@@ -920,7 +920,7 @@ static cudaError_t launch_topk_groups(const float *scores, PageOut page_list, in
                                       int n_pages, int k, cudaStream_t stream) {
     const int cap = topk_candidate_capacity(k);      // at most 2048 here: 24 KB, no opt-in needed
     const size_t smem = (size_t)(cap + 2) * sizeof(unsigned long long) + (size_t)cap * sizeof(int);
-    const cudaError_t e = launch_dependent(topk_pages_groups_kernel<PER, VEC>, dim3(rows), dim3(kTopkThreads), smem, stream,
+    const cudaError_t e = launch_dependent_at(kChainPriority, topk_pages_groups_kernel<PER, VEC>, dim3(rows), dim3(kTopkThreads), smem, stream,
                                            scores, page_list, n_kv_heads, rep, n_pages, k);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
