@@ -636,8 +636,8 @@ static size_t lru_smem_bytes(int n_slots, int list_len) {
 }
 
 static size_t lru_queue_smem_bytes(int n_slots, int list_len) {
-    return ((size_t)2 * lru_table_size(list_len) + 2 * (size_t)list_len) * sizeof(int) +
-           (((size_t)n_slots + 15) & ~(size_t)15);   // a multiple of 16: the page staging area follows
+    const size_t tables = ((size_t)2 * lru_table_size(list_len) + 2 * (size_t)list_len) * sizeof(int) + (size_t)n_slots;
+    return (tables + 15) & ~(size_t)15;   // the page staging area follows: bulk copies and 16-byte loads, also for an odd list_len
 }
 
 constexpr size_t kLruMaxSmem = 227 * 1024 - 4096;

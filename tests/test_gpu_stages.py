@@ -365,6 +365,28 @@ def test_lru_random_trajectories_bit_exact(da, hk, ld, nh, kk, steps, page_dim, 
     assert int(t.g_status) == 0
 
 
+@pytest.mark.parametrize("kk,nh", [(1, 4), (3, 17), (15, 60), (103, 207), (1023, 2047), (1025, 4095)])
+def test_lru_update_copies_pages_of_an_odd_list(da, kk, nh):
+    """An odd number of listed pages (one query head with an odd k): the tables in shared memory then end between two
+    16-byte boundaries, and the pages the update copies itself are staged behind them on the next one."""
+    rng = np.random.default_rng(kk)
+    t = Tables(2, 3 * nh, nh, page_dim=64, dtype=torch.bfloat16, seed=kk).to_device()
+    resident = [np.flatnonzero(t.d2h[h] >= 0) for h in range(2)]
+    for s in range(4):
+        lst = np.stack([rng.choice(r, size=kk) for r in resident])
+        fresh = min(kk, 6)                                   # as many misses as the call copies itself
+        lst[:, rng.permutation(kk)[:fresh]] = rng.choice(np.arange(3 * nh), size=(2, fresh), replace=False)
+        mp_c, ms_c, nm_c = t.cpu_step(lst)
+        mp_g, ms_g, nm_g = t.gpu_step(lst, use_queue=True, inline=6)
+        assert np.array_equal(nm_g, nm_c), s
+        for h in range(2):
+            assert np.array_equal(mp_g[h, :nm_c[h]], mp_c[h, :nm_c[h]]), (s, h)
+            assert np.array_equal(ms_g[h, :nm_c[h]], ms_c[h, :nm_c[h]]), (s, h)
+        t.assert_equal(f"step {s}")
+        resident = [np.flatnonzero(t.d2h[h] >= 0) for h in range(2)]
+    assert int(t.g_status) == 0
+
+
 def test_lru_overflow_and_bad_page_are_reported(da):
     t = Tables(1, 16, 4).to_device()
     lst = np.array([[0, 1, 2, 3, 4, 5]])  # 6 distinct non-resident pages, 4 slots
