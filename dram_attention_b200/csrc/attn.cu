@@ -182,19 +182,19 @@ struct SimtMath {
 // Warps per CTA: as many as the shared memory of an SM holds stages for (float32 units are twice as large).
 template <typename M> __host__ __device__ constexpr int simt_warps() { return M::kStages * M::UNITB > 24576 ? 6 : 8; }
 
-template <typename T, int D, int ROWS>
+template <typename T, int D, int ROWS, bool TWO>
 __global__ void __launch_bounds__(simt_warps<SimtMath<T, D, ROWS>>() * 32, 1) decode_attention_kernel(const AttnParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     using M = SimtMath<T, D, ROWS>;
-    decode_attention_body<M, simt_warps<M>(), M::kStages>(p, smem);
+    decode_attention_body<M, simt_warps<M>(), M::kStages, TWO>(p, smem);
 }
 
-template <typename T, int D, int ROWS>
-static cudaError_t launch_attn(const AttnParams &p, int n_kv_heads, int splits, cudaStream_t stream) {
+template <typename T, int D, int ROWS, bool TWO>
+static cudaError_t launch_attn_as(const AttnParams &p, int n_kv_heads, int splits, cudaStream_t stream) {
     using M = SimtMath<T, D, ROWS>;
     constexpr int WARPS = simt_warps<M>();
     constexpr int SMEM = WARPS * M::kStages * M::UNITB;
-    auto kern = decode_attention_kernel<T, D, ROWS>;
+    auto kern = decode_attention_kernel<T, D, ROWS, TWO>;
     static bool attr_set[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -211,6 +211,12 @@ static cudaError_t launch_attn(const AttnParams &p, int n_kv_heads, int splits, 
     if (p.phase != 1) return launch_dependent_at(p.phase == 2 ? kChainPriority : 0, kern, grid, dim3(WARPS * 32), (size_t)SMEM, stream, p);
     kern<<<grid, WARPS * 32, SMEM, stream>>>(p);
     return cudaGetLastError();
+}
+
+template <typename T, int D, int ROWS>
+static cudaError_t launch_attn(const AttnParams &p, int n_kv_heads, int splits, cudaStream_t stream) {
+    return p.phase != 0 ? launch_attn_as<T, D, ROWS, true>(p, n_kv_heads, splits, stream)
+                        : launch_attn_as<T, D, ROWS, false>(p, n_kv_heads, splits, stream);
 }
 
 // float32: up to 8 query rows per launch (register budget)

@@ -28,7 +28,6 @@ constexpr int kPrefetchUnits = 2;
 constexpr unsigned int kTicketPhase2 = 1u << 12;     // a CTA of phase 2 (a launch has at most kAttnMaxSplits per head)
 constexpr unsigned int kTicketMerged = 1u << 30;     // phase 1's partials have been merged into one
 static_assert(kAttnMaxSplits < (int)kTicketPhase2, "the counts of the two launches stay apart");
-enum { kMergeNothing, kMergePhase1, kMergeAll, kMergeRest };
 
 __device__ __forceinline__ unsigned int take_ticket(unsigned int *word, unsigned int add) {
     unsigned int old;
@@ -36,7 +35,8 @@ __device__ __forceinline__ unsigned int take_ticket(unsigned int *word, unsigned
     return old;
 }
 
-template <typename Math, int WARPS, int STAGES>
+// TWO: one of two launches (their final merge is code of its own).
+template <typename Math, int WARPS, int STAGES, bool TWO>
 __device__ __forceinline__ void decode_attention_body(const AttnParams &p, unsigned char *smem) {
     using T = typename Math::Elem;
     constexpr int D = Math::kD;
@@ -305,11 +305,11 @@ __device__ __forceinline__ void decode_attention_body(const AttnParams &p, unsig
     }
     if (todo == kMergeNothing) return;
 
-    if (todo == kMergePhase1) {
-        // ---- the last CTA of phase 1, phase 2 still at work: phase 1's partials become one, so that the merge at the
-        //      end of the step has only phase 2's few beside it (8 rows of 44 partials: 5.4 us, of 7: 3.1) ------
-        merge_partials<T, D, THREADS>(p, h, 0, p.splits1, rows, nullptr,
-                                      p.partials + ((size_t)(h * p.part_rows + p.ticket_target) * rows) * PW, smem);
+    // kMergePhase1: the last CTA of phase 1, phase 2 still at work; with phase 1's partials in one, the merge at the end of the
+    // step has only phase 2's few beside it (8 rows of 44 partials: 5.4 us, of 7: 3.1).  Otherwise this CTA of the head
+    // finished last (of both launches, when there are two) and writes the output.
+    merge_partials<T, D, THREADS, TWO>(p, h, rows, todo, smem);
+    if (TWO && todo == kMergePhase1) {
         __syncthreads();
         if (tid == 0) {
             // Said in the ticket word, where the last CTA reads it with its ticket.  A word that is zero again means
@@ -320,11 +320,6 @@ __device__ __forceinline__ void decode_attention_body(const AttnParams &p, unsig
         return;
     }
 
-    // ---- the CTA of this head that finished last (of both launches, when there are two) --------
-    // a head that phase 2 redid: phase 1's rows (the first in the workspace, or merged into the one behind all) are left out
-    const bool rest = todo == kMergeRest;
-    merge_partials<T, D, THREADS>(p, h, rest ? p.splits1 : 0, p.ticket_target + (rest ? 1 : 0), rows,
-                                  p.phase != 0 ? p.redo + h : nullptr, nullptr, smem);
     // every CTA of this head is done with the eviction front: the one the LRU update left becomes current
     if (p.phase != 0 && tid == 0) atomicXor(p.flip + h, 1);   // (no result wanted: the CTA does not wait for it)
     if (tid == 0) asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p.counters + h), "r"(0u) : "memory");

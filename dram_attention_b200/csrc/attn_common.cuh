@@ -25,7 +25,9 @@ constexpr int kRoundUnits = 32;        // units a warp plans at a time (one per 
 // Phase 1 runs beside the selection kernels, whose CTAs need a whole SM each: it has at most 116 CTAs, so that
 // wherever the hardware places them 32 of the 148 SMs stay empty.  Phase 2 covers the few slots the LRU update
 // could evict, on what phase 1 and the update's CTAs (one per head) leave.  The caps on CTAs per head keep the merge
-// at one batch per thread (4 query rows: 3 x 18 partials); the single launch also keeps at least two units per warp.
+// short: of 4 query rows of 128 channels a thread has at most 16 partials of phase 1 (two batches) and two of phase 2, of 8
+// rows (one group of threads instead of three) of three heads 38 and 6.  The single launch also keeps at least two units
+// per warp.
 constexpr int kAttnPhase1Ctas = 116;
 constexpr int kAttnPhase1MaxPerHead = 48;
 constexpr int kAttnPhase2MaxPerHead = 6;
@@ -255,155 +257,217 @@ __device__ __forceinline__ int plan_commit(const AttnParams &p, const LaunchUnit
 // be read with 128-bit loads.
 template <int D> struct PartialRow { static constexpr int kWidth = D + 4; };
 
-// Running softmax merge of (max, l, four accumulator columns); log2 domain.
+// Running softmax merge of (max, l, four accumulator columns); log2 domain.  Every product and sum is spelled out, so that
+// the same operands give the same bits wherever this is compiled in.
 struct MergeAcc {
     float m, l;
     float4 a;
 };
+__device__ __forceinline__ MergeAcc merge_nothing() { return {-INFINITY, 0.f, make_float4(0.f, 0.f, 0.f, 0.f)}; }
 __device__ __forceinline__ void merge_into(MergeAcc &x, float m, float l, const float4 &v) {
     const float mn = fmaxf(x.m, m);
     const float ms = (mn == -INFINITY) ? 0.f : mn;
     const float wx = fast_exp2(x.m - ms), wv = fast_exp2(m - ms);
     x.m = mn;
-    x.l = x.l * wx + l * wv;
-    x.a.x = x.a.x * wx + v.x * wv;
-    x.a.y = x.a.y * wx + v.y * wv;
-    x.a.z = x.a.z * wx + v.z * wv;
-    x.a.w = x.a.w * wx + v.w * wv;
+    x.l = fmaf(x.l, wx, __fmul_rn(l, wv));
+    x.a.x = fmaf(x.a.x, wx, __fmul_rn(v.x, wv));
+    x.a.y = fmaf(x.a.y, wx, __fmul_rn(v.y, wv));
+    x.a.z = fmaf(x.a.z, wx, __fmul_rn(v.z, wv));
+    x.a.w = fmaf(x.a.w, wx, __fmul_rn(v.w, wv));
 }
 
-// Merge of the per-CTA partials [lo, hi) of one head by one CTA of THREADS threads.  A CTA's partial = `rows` rows
+// What a CTA adds up once its ticket is taken: nothing, phase 1's partials into one (phase 2 is still at work), or the
+// head's output from all partials, or from phase 2's and the one that phase 1's were merged into.
+enum { kMergeNothing, kMergePhase1, kMergeAll, kMergeRest };
+
+// Partials of every `step`-th CTA from s0 on, requested together (the last one again for places behind the end).
+template <int BATCH> struct PartialBatch {
+    float4 v[BATCH];
+    float2 w[BATCH];
+    __device__ __forceinline__ void request(const float *col, const float *ml, size_t cta_stride, int s0, int step, int hi) {
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i) {
+            const int s = min(s0 + i * step, hi - 1);
+            v[i] = __ldcg(reinterpret_cast<const float4 *>(col + (size_t)s * cta_stride));
+            w[i] = __ldcg(reinterpret_cast<const float2 *>(ml + (size_t)s * cta_stride));
+        }
+    }
+    // The batch's own maximum first, so that its exponentials do not wait for one another.
+    __device__ __forceinline__ void fold_into(MergeAcc &x, int s0, int step, int hi, bool skip) {
+        float mb = x.m;
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i) {
+            if (skip || s0 + i * step >= hi) w[i].x = -INFINITY;
+            mb = fmaxf(mb, w[i].x);
+        }
+        const float ms = (mb == -INFINITY) ? 0.f : mb;
+        const float wx = fast_exp2(x.m - ms);
+        x.m = mb;
+        x.l = __fmul_rn(x.l, wx);
+        x.a.x = __fmul_rn(x.a.x, wx);
+        x.a.y = __fmul_rn(x.a.y, wx);
+        x.a.z = __fmul_rn(x.a.z, wx);
+        x.a.w = __fmul_rn(x.a.w, wx);
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i) {
+            if (w[i].x == -INFINITY) continue;   // (a CTA without units: its rows are zeros)
+            const float wv = fast_exp2(w[i].x - ms);
+            x.l = fmaf(w[i].y, wv, x.l);
+            x.a.x = fmaf(v[i].x, wv, x.a.x);
+            x.a.y = fmaf(v[i].y, wv, x.a.y);
+            x.a.z = fmaf(v[i].z, wv, x.a.z);
+            x.a.w = fmaf(v[i].w, wv, x.a.w);
+        }
+    }
+};
+
+template <int BATCH>
+__device__ __forceinline__ void fold_partials(MergeAcc &x, const float *col, const float *ml, size_t cta_stride, int lo, int step,
+                                              int hi, bool skip) {
+    for (int s0 = lo; s0 < hi; s0 += step * BATCH) {
+        PartialBatch<BATCH> b;
+        b.request(col, ml, cta_stride, s0, step, hi);
+        b.fold_into(x, s0, step, hi, skip);
+    }
+}
+
+// Merge of the per-CTA partials of one head by one CTA of THREADS threads.  A CTA's partial = `rows` rows
 // of (acc[D] already weighted to the row's max, max, l); the partials of consecutive CTAs are contiguous in the
 // workspace.  It is on the critical path of every step and bound by latency alone, so it is one round trip to
 // L2 wherever the registers allow: a thread owns four columns of a row for every G-th CTA (G = how many
 // times the row-columns fit into the CTA), requests BATCH partials together with their (max, l) pairs, and
 // folds them in registers; the G groups meet in shared memory.  (Staging the rows in shared memory in two
-// halves, as before, took one round trip per half: 3.7 us for 22 partials of 4 rows, 5.9 us for 55.)
-// `merged` (may be null): where the result goes as one more partial; otherwise it is the head's output.
-// `skip_flag` (may be null): when the word it points to is non-zero phase 1's partials, and the one they were
-// merged into, are left out.
+// halves took one round trip per half: 3.7 us for 22 partials of 4 rows, 5.9 us for 55.)
+// With two launches phase 1's partials and phase 2's are always added up apart and the two sums put together at the
+// end: the output's bits do not depend on which launch was through first, i.e. on whether phase 1's own last CTA has
+// done its part already (kMergeRest) or not (kMergeAll).  A head that phase 2 redid leaves phase 1's partials out.
 // With kMergeBatchFew partials per thread or less a short batch: the long one asks for the last partial again and
-// again (four resident 13K layers 78.3 / 74.0 us).
+// again (four resident 13K layers 78.3 / 74.0 us).  With two launches the long one is no longer than 9, and one piece of
+// code serves every case: it runs once or twice per head and layer, on an SM that seldom has it at hand, so its size
+// counts as much as another round trip.  us for three odd 77K layers (38 partials of 8 rows in phase 1) / four 128K layers:
+// long batch of 18, 12, 9: 84 / 167, 83 / 166, 81.5 / 165.4; with every case's code apart 85 / 166; a batch of 9 in kernels
+// that hold no other launch's merge 77 / 165.8 (and four resident 13K layers 73.8 instead of 75.2).
 constexpr int kMergeBatch = 18;
+constexpr int kMergeBatchTwo = 9;
 constexpr int kMergeBatchFew = 6;
 
-template <typename T, int D, int THREADS, int BATCH>
-__device__ __forceinline__ void merge_range(const AttnParams &p, int h, int lo, int hi, int rows, const int32_t *skip_flag,
-                                            float *merged, unsigned char *smem) {
+// TWO: the kernel is one of two launches.
+template <typename T, int D, int THREADS, int BATCH, bool TWO>
+__device__ __forceinline__ void merge_partials_by(const AttnParams &p, int h, int rows, int todo, unsigned char *smem) {
+    const bool with1 = !TWO || todo != kMergeRest;        // add up phase 1's (a single launch's) partials
+    const bool with2 = TWO && todo != kMergePhase1;       // ... phase 2's, requested ahead of a short batch of phase 1's
+    constexpr bool ahead2 = TWO && BATCH <= kMergeBatchFew;
     constexpr int PW = PartialRow<D>::kWidth;
     constexpr int VPR = D / 4;          // float4 per accumulator row
     const int tid = threadIdx.x;
     const int32_t peer_step = p.peer_world > 0 ? __ldcg(p.peer_seq) : 0;   // (needed at the very end: read now)
-    const bool skip = skip_flag != nullptr && __ldcg(skip_flag) != 0;
+    const bool skip = with2 && __ldcg(p.redo + h) != 0;
+    const int n1 = TWO ? p.splits1 : p.ticket_target, n = p.ticket_target;
     const float *hp = p.partials + ((size_t)h * p.part_rows * rows) * PW;
+    float *merged1 = p.partials + ((size_t)(h * p.part_rows + n) * rows) * PW;   // phase 1's, once merged
     const size_t cta_stride = (size_t)rows * PW;
     const int items = rows * VPR;
     const int groups = max(THREADS / items, 1);
-    float4 *sh_a = reinterpret_cast<float4 *>(smem);                    // [groups - 1][items]
-    float2 *sh_ml = reinterpret_cast<float2 *>(sh_a + THREADS);         // [groups - 1][items]
+    float4 *sh_a = reinterpret_cast<float4 *>(smem);                    // [2][groups - 1][items]
+    float2 *sh_ml = reinterpret_cast<float2 *>(sh_a + 2 * THREADS);     // [2][groups - 1][items]
     const int g = groups > 1 ? tid / items : 0;
 
     for (int e0 = 0; e0 < items; e0 += THREADS) {
         const int e = groups > 1 ? tid % items : e0 + tid;
         const bool mine = e < items && g < groups;
-        MergeAcc x = {-INFINITY, 0.f, make_float4(0.f, 0.f, 0.f, 0.f)};
+        const size_t at = (size_t)(e / VPR) * PW + 4 * (e % VPR), at_ml = (size_t)(e / VPR) * PW + D;
+        MergeAcc x1 = merge_nothing(), x2 = merge_nothing();
         if (mine) {
-            const float *col = hp + (size_t)(e / VPR) * PW + 4 * (e % VPR);
-            const float *ml = hp + (size_t)(e / VPR) * PW + D;
-            for (int s0 = lo + g; s0 < hi; s0 += groups * BATCH) {
-                float4 v[BATCH];
-                float2 w[BATCH];
-#pragma unroll
-                for (int i = 0; i < BATCH; ++i) {
-                    const int s = min(s0 + i * groups, hi - 1);
-                    v[i] = __ldcg(reinterpret_cast<const float4 *>(col + (size_t)s * cta_stride));
-                    w[i] = __ldcg(reinterpret_cast<const float2 *>(ml + (size_t)s * cta_stride));
-                }
-                // the batch's own maximum first, so that its exponentials do not wait for one another
-                float mb = x.m;
-#pragma unroll
-                for (int i = 0; i < BATCH; ++i) {
-                    const int s = s0 + i * groups;
-                    if (s >= hi || (skip && (s < p.splits1 || s == p.ticket_target))) w[i].x = -INFINITY;
-                    mb = fmaxf(mb, w[i].x);
-                }
-                const float ms = (mb == -INFINITY) ? 0.f : mb;
-                const float wx = fast_exp2(x.m - ms);
-                x.m = mb;
-                x.l *= wx;
-                x.a.x *= wx; x.a.y *= wx; x.a.z *= wx; x.a.w *= wx;
-#pragma unroll
-                for (int i = 0; i < BATCH; ++i) {
-                    if (w[i].x == -INFINITY) continue;   // (a CTA without units: its rows are zeros)
-                    const float wv = fast_exp2(w[i].x - ms);
-                    x.l = fmaf(w[i].y, wv, x.l);
-                    x.a.x = fmaf(v[i].x, wv, x.a.x);
-                    x.a.y = fmaf(v[i].y, wv, x.a.y);
-                    x.a.z = fmaf(v[i].z, wv, x.a.z);
-                    x.a.w = fmaf(v[i].w, wv, x.a.w);
-                }
+            const float *col = hp + at, *ml = hp + at_ml;
+            PartialBatch<ahead2 ? kMergeBatchFew : 1> b2;
+            if (ahead2 && with2) b2.request(col, ml, cta_stride, n1 + g, groups, n);
+            if (with1) {
+                fold_partials<BATCH>(x1, col, ml, cta_stride, g, groups, n1, skip);
+            } else if (g == 0) {
+                const float4 v = __ldcg(reinterpret_cast<const float4 *>(merged1 + at));   // (set out before `skip` is there)
+                const float2 w = __ldcg(reinterpret_cast<const float2 *>(merged1 + at_ml));
+                if (!skip) x1 = {w.x, w.y, v};
             }
+            if (ahead2 && with2) b2.fold_into(x2, n1 + g, groups, n, false);
+            if (with2)
+                fold_partials<kMergeBatchFew>(x2, col, ml, cta_stride, n1 + g + (ahead2 ? groups * kMergeBatchFew : 0), groups, n, false);
         }
         if (groups > 1) {
+            const int half = (groups - 1) * items;
             if (mine && g > 0) {
-                sh_a[(g - 1) * items + e] = x.a;
-                sh_ml[(g - 1) * items + e] = make_float2(x.m, x.l);
+                const int at_sh = (g - 1) * items + e;
+                if (with1) {
+                    sh_a[at_sh] = x1.a;
+                    sh_ml[at_sh] = make_float2(x1.m, x1.l);
+                }
+                if (with2) {
+                    sh_a[half + at_sh] = x2.a;
+                    sh_ml[half + at_sh] = make_float2(x2.m, x2.l);
+                }
             }
             __syncthreads();
             if (mine && g == 0) {
                 for (int k = 0; k < groups - 1; ++k) {
-                    const float2 w = sh_ml[k * items + e];
-                    merge_into(x, w.x, w.y, sh_a[k * items + e]);
+                    const int at_sh = k * items + e;
+                    if (with1) merge_into(x1, sh_ml[at_sh].x, sh_ml[at_sh].y, sh_a[at_sh]);
+                    if (with2) merge_into(x2, sh_ml[half + at_sh].x, sh_ml[half + at_sh].y, sh_a[half + at_sh]);
                 }
             }
         }
-        if (mine && g == 0 && merged != nullptr) {
-            const int r = e / VPR, c4 = e % VPR;
-            *reinterpret_cast<float4 *>(merged + (size_t)r * PW + 4 * c4) = x.a;
-            if (c4 == 0) *reinterpret_cast<float2 *>(merged + (size_t)r * PW + D) = make_float2(x.m, x.l);
-        } else if (mine && g == 0) {
-            const int r = e / VPR, c4 = e % VPR;
-            const float inv = x.l > 0.f ? 1.f / x.l : 0.f;
-            // row r = (query token, head of the group)
-            const int tok = p.q_tok0 + r / p.rep;
-            const size_t orow = (size_t)tok * p.n_kv_heads * p.rep + (size_t)h * p.rep + r % p.rep;
-            union { T t[4]; uint32_t w[sizeof(T)]; } o;   // four elements as whole words (2 or 4 of them)
-            o.t[0] = from_float<T>(x.a.x * inv);
-            o.t[1] = from_float<T>(x.a.y * inv);
-            o.t[2] = from_float<T>(x.a.z * inv);
-            o.t[3] = from_float<T>(x.a.w * inv);
-            T *dst = reinterpret_cast<T *>(p.out) + orow * D + 4 * c4;
-            if constexpr (sizeof(T) == 4) *reinterpret_cast<uint4 *>(dst) = make_uint4(o.w[0], o.w[1], o.w[2], o.w[3]);
-            else *reinterpret_cast<uint2 *>(dst) = make_uint2(o.w[0], o.w[1]);
-            if (c4 == 0 && p.lse_out)
-                p.lse_out[orow] = ((x.m == -INFINITY ? 0.f : x.m) + log2f(x.l)) * 0.6931471805599453f;
-            if (p.peer_world > 0) {
-                // these four values as payload words {payload, tag} into slot (seq & 1) of every rank's buffer,
-                // at this rank's place (one query token per call: orow is the head row)
-                const int32_t sq = peer_step;
-                const uint32_t tag = (uint32_t)(sq + 1);
-                constexpr int NW = (int)sizeof(T);
-                const size_t word0 = (size_t)(sq & 1) * p.peer_world * p.peer_words + (size_t)p.peer_rank * p.peer_words +
-                                     (orow * D + 4 * c4) * sizeof(T) / 4;
+        if (!mine || g != 0) continue;
+        const int r = e / VPR, c4 = e % VPR;
+        if (TWO && todo == kMergePhase1) {
+            *reinterpret_cast<float4 *>(merged1 + at) = x1.a;
+            if (c4 == 0) *reinterpret_cast<float2 *>(merged1 + at_ml) = make_float2(x1.m, x1.l);
+            continue;
+        }
+        if (with2) {
+            merge_into(x2, x1.m, x1.l, x1.a);
+            x1 = x2;
+        }
+        const float inv = x1.l > 0.f ? 1.f / x1.l : 0.f;
+        // row r = (query token, head of the group)
+        const int tok = p.q_tok0 + r / p.rep;
+        const size_t orow = (size_t)tok * p.n_kv_heads * p.rep + (size_t)h * p.rep + r % p.rep;
+        union { T t[4]; uint32_t w[sizeof(T)]; } o;   // four elements as whole words (2 or 4 of them)
+        o.t[0] = from_float<T>(x1.a.x * inv);
+        o.t[1] = from_float<T>(x1.a.y * inv);
+        o.t[2] = from_float<T>(x1.a.z * inv);
+        o.t[3] = from_float<T>(x1.a.w * inv);
+        T *dst = reinterpret_cast<T *>(p.out) + orow * D + 4 * c4;
+        if constexpr (sizeof(T) == 4) *reinterpret_cast<uint4 *>(dst) = make_uint4(o.w[0], o.w[1], o.w[2], o.w[3]);
+        else *reinterpret_cast<uint2 *>(dst) = make_uint2(o.w[0], o.w[1]);
+        if (c4 == 0 && p.lse_out)
+            p.lse_out[orow] = ((x1.m == -INFINITY ? 0.f : x1.m) + log2f(x1.l)) * 0.6931471805599453f;
+        if (p.peer_world > 0) {
+            // these four values as payload words {payload, tag} into slot (seq & 1) of every rank's buffer,
+            // at this rank's place (one query token per call: orow is the head row)
+            const int32_t sq = peer_step;
+            const uint32_t tag = (uint32_t)(sq + 1);
+            constexpr int NW = (int)sizeof(T);
+            const size_t word0 = (size_t)(sq & 1) * p.peer_world * p.peer_words + (size_t)p.peer_rank * p.peer_words +
+                                 (orow * D + 4 * c4) * sizeof(T) / 4;
 #pragma unroll
-                for (int gp = 0; gp < kAttnMaxPeers; ++gp) {
-                    if (gp < p.peer_world) {
-                        uint2 *pd = p.peer_buf[gp] + word0;
+            for (int gp = 0; gp < kAttnMaxPeers; ++gp) {
+                if (gp < p.peer_world) {
+                    uint2 *pd = p.peer_buf[gp] + word0;
 #pragma unroll
-                        for (int i = 0; i < NW; ++i) st_word_sys(pd + i, o.w[i], tag);
-                    }
+                    for (int i = 0; i < NW; ++i) st_word_sys(pd + i, o.w[i], tag);
                 }
             }
         }
     }
 }
 
-template <typename T, int D, int THREADS>
-__device__ __forceinline__ void merge_partials(const AttnParams &p, int h, int lo, int hi, int rows,
-                                               const int32_t *skip_flag, float *merged, unsigned char *smem) {
+template <typename T, int D, int THREADS, bool TWO>
+__device__ __forceinline__ void merge_partials(const AttnParams &p, int h, int rows, int todo, unsigned char *smem) {
+    constexpr int LONG = TWO ? kMergeBatchTwo : kMergeBatch;
     const int groups = max(THREADS / (rows * (D / 4)), 1);
-    if (hi - lo <= kMergeBatchFew * groups) merge_range<T, D, THREADS, kMergeBatchFew>(p, h, lo, hi, rows, skip_flag, merged, smem);
-    else merge_range<T, D, THREADS, kMergeBatch>(p, h, lo, hi, rows, skip_flag, merged, smem);
+    const int n1 = TWO ? p.splits1 : p.ticket_target;
+    if ((TWO && todo == kMergeRest) || n1 <= kMergeBatchFew * groups)
+        merge_partials_by<T, D, THREADS, kMergeBatchFew, TWO>(p, h, rows, todo, smem);
+    else
+        merge_partials_by<T, D, THREADS, LONG, TWO>(p, h, rows, todo, smem);
 }
 
 // 16-bit element types: tensor-core kernel (attn_mma.cu).

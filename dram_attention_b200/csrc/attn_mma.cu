@@ -397,16 +397,16 @@ struct MmaMathWide {
 constexpr int kMmaWideWarps = 8, kMmaWideStages = 3;
 constexpr int kMmaStages = 2;   // per warp: 12 x 2 stages are 203 KB of an SM's shared memory for head_dim 128
 
-template <typename T, int D, bool FULL>
+template <typename T, int D, bool FULL, bool TWO>
 __global__ void __launch_bounds__(kAttnWarps * 32, 1) decode_attention_mma_kernel(const AttnParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    decode_attention_body<MmaMath<T, D, FULL>, kAttnWarps, kMmaStages>(p, smem);
+    decode_attention_body<MmaMath<T, D, FULL>, kAttnWarps, kMmaStages, TWO>(p, smem);
 }
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kMmaWideWarps * 32, 1) decode_attention_mma_wide_kernel(const AttnParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    decode_attention_body<MmaMathWide<T, D>, kMmaWideWarps, kMmaWideStages>(p, smem);
+    decode_attention_body<MmaMathWide<T, D>, kMmaWideWarps, kMmaWideStages, false>(p, smem);
 }
 
 template <typename T, int D, int WARPS, int SMEM, void (*kern)(const AttnParams)>
@@ -435,8 +435,11 @@ static cudaError_t launch_mma_d(const AttnParams &p, int n_kv_heads, int splits,
     constexpr int kSmem = kAttnWarps * kMmaStages * kStageBytes, kWideSmem = kMmaWideWarps * kMmaWideStages * kStageBytes;
     const int rows = p.n_q * p.rep;
     if (rows > 16) return launch_mma<T, D, kMmaWideWarps, kWideSmem, decode_attention_mma_wide_kernel<T, D>>(p, n_kv_heads, splits, stream);
-    if (rows > 8) return launch_mma<T, D, kAttnWarps, kSmem, decode_attention_mma_kernel<T, D, true>>(p, n_kv_heads, splits, stream);
-    return launch_mma<T, D, kAttnWarps, kSmem, decode_attention_mma_kernel<T, D, false>>(p, n_kv_heads, splits, stream);
+    const bool two = p.phase != 0;
+    if (rows > 8 && two) return launch_mma<T, D, kAttnWarps, kSmem, decode_attention_mma_kernel<T, D, true, true>>(p, n_kv_heads, splits, stream);
+    if (rows > 8) return launch_mma<T, D, kAttnWarps, kSmem, decode_attention_mma_kernel<T, D, true, false>>(p, n_kv_heads, splits, stream);
+    if (two) return launch_mma<T, D, kAttnWarps, kSmem, decode_attention_mma_kernel<T, D, false, true>>(p, n_kv_heads, splits, stream);
+    return launch_mma<T, D, kAttnWarps, kSmem, decode_attention_mma_kernel<T, D, false, false>>(p, n_kv_heads, splits, stream);
 }
 
 template <typename T>

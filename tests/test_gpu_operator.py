@@ -732,3 +732,92 @@ def test_two_launch_merge_at_any_number_of_partials(da, ctas1, ctas2, rep, dtype
     assert a._can_overlap and a._overlap_supported(rep, dtype)
     for m in (a, b):
         m.check_status()
+
+
+def _two_launch_operators(da, n, hk, rep, d, dtype, steps, redraw):
+    """n operators in the same state after `steps` calls, and the inputs of the next one."""
+    g = torch.Generator().manual_seed(hk * 100 + rep + d)
+    length, page = 6000, 16
+    k, v = (torch.randn(1, length, hk, d, generator=g).to(dtype).to(DEV) for _ in range(2))
+    u = torch.randn(hk * rep, d, generator=g)
+    ms = [da.DRAMAttention(max_output_length=steps + 4, lru_hbm_cache_size=1536, local_cache_size=300, page_size=page,
+                           top_k=page * max(1, 60 // rep), n_kv_heads=hk, head_dim=d, device=DEV, dtype=dtype)
+          for _ in range(n)]
+    for m in ms:
+        m.init_cache(k, v)
+    for i in range(steps + 1):
+        q = u + 0.1 * torch.randn(hk * rep, d, generator=g)
+        if redraw and i == steps:
+            q = torch.randn(hk * rep, d, generator=g)
+        x = [q.to(dtype).to(DEV).view(1, 1, -1, d)]
+        x += [torch.randn(1, 1, hk, d, generator=g).to(dtype).to(DEV) for _ in range(2)]
+        if i < steps:
+            for m in ms:
+                m(*x, start_pos=length + i, stage="generate")
+    assert ms[0]._can_overlap and ms[0]._overlap_supported(rep, dtype)
+    return ms, x, length + steps
+
+
+@pytest.mark.parametrize("ctas1,ctas2", [(0, 0), (1, 1), (2, 5), (3, 1), (48, 7), (148, 148)])
+@pytest.mark.parametrize("hk,rep,d,dtype", [(2, 4, 128, torch.bfloat16), (3, 8, 128, torch.float16), (2, 1, 64, torch.bfloat16),
+                                            (2, 4, 64, torch.float32), (1, 8, 64, torch.float32)])
+@pytest.mark.parametrize("redraw", [False, True])
+def test_output_bits_do_not_depend_on_which_launch_ends_first(da, ctas1, ctas2, hk, rep, d, dtype, redraw):
+    """One step of the two-launch layout with phase 1 through before phase 2 starts (its partials are merged in advance), with
+    phase 2 through before phase 1 starts, and with phase 1 first in a workspace that has no room for merging in
+    advance: outputs and log-sum-exps are equal to the bit, also for heads that phase 2 redoes."""
+    ms, x, pos = _two_launch_operators(da, 3, hk, rep, d, dtype, 3, redraw)
+    outs = []
+    for order, m in enumerate(ms):
+        m.phase1_ctas, m.phase2_ctas = ctas1, ctas2
+        lc = m.lru_cache
+        out, lse = torch.empty_like(x[0]), torch.empty(hk * rep, device=DEV)
+        buf, nbytes, status = m._workspace(rep, out.device)
+        if order == 2:
+            splits1 = ctas1 or da._native.lib().da_decode_attention_phase1_ctas(hk)
+            splits2 = ctas2 or min(6, (148 - hk * (splits1 + 1)) // hk)
+            m._ws[(rep, 1)] = (buf, 1024 + hk * (splits1 + splits2) * rep * (d + 4) * 4, status)
+        _, page_list = lc.top_k_selector.page_list_(x[0], lc.top_k)
+        torch.cuda.synchronize()
+        phase = lambda n: (m.attend_(*x, pos, out, lse=lse, phase=n), torch.cuda.synchronize())
+        if order != 1:
+            phase(1)
+        lc.update_tables_(page_list, advance_split=False, inline_fetch=True)
+        phase(2)
+        if order == 1:
+            phase(1)
+        assert bool(lc.evict_redo[0].any()) == redraw or not redraw
+        assert not bool(buf[:1024].any())
+        m.check_status()
+        outs.append((out, lse))
+    for out, lse in outs[1:]:
+        assert torch.equal(out, outs[0][0]) and torch.equal(lse, outs[0][1])
+
+
+@pytest.mark.parametrize("hk,rep,d,dtype", [(8, 4, 128, torch.bfloat16), (2, 4, 64, torch.float32)])
+def test_two_launch_step_repeats_bit_for_bit(da, hk, rep, d, dtype):
+    """A captured step replayed many times from one saved state, alone and beside other work on the GPU."""
+    (m,), x, pos = _two_launch_operators(da, 1, hk, rep, d, dtype, 3, False)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        out = m(*x, start_pos=pos, stage="generate")
+    state = [t for n, t in m.lru_cache.named_buffers() if n != "dram_kv_cache"]
+    state += [m.cache_k, m.cache_v] + [w[0] for w in m._ws.values()]
+    saved = [t.clone() for t in state]
+    a = torch.randn(2048, 2048, device=DEV)
+    other = torch.cuda.Stream()
+    outs = []
+    for i in range(24):
+        for t, s in zip(state, saved):
+            t.copy_(s)
+        torch.cuda.synchronize()
+        if i % 3:
+            with torch.cuda.stream(other):
+                for _ in range(i):
+                    a @ a
+        graph.replay()
+        torch.cuda.synchronize()
+        outs.append(out.clone())
+    assert all(torch.equal(outs[0], o) for o in outs[1:])
+    m.check_status()
