@@ -672,8 +672,10 @@ topk_pages_cluster_kernel(const float *__restrict__ scores, PageOut page_list, i
 // once: a thread keeps the maxima of kGroups groups of 4 * PER scores.  The k-th largest of all group maxima is a
 // lower bound of the k-th largest score (k groups hold at least one score each that reaches it), so the
 // selected pages lie in the groups whose maximum reaches the bucket of that bound: a few more than k of them, which
-// are read a second time.  Bound by latency: 2.5 us for the row out of L2, then five dependent stages.  Their scores from that bucket on are the candidates, sorted by bucket and
-// ranked inside their bucket as in the kernel above.  Rows this cannot resolve (NaN, constant rows, massive
+// are read a second time.  Bound by latency: 2.5 us for the row out of L2, then five dependent stages.  Their scores
+// from the bucket of the k-th on are the candidates, sorted by bucket and ranked inside their bucket as in the kernel
+// above.  That bucket is found among the scores read again, not among the maxima: where neighbouring pages score alike
+// (as text does) whole groups qualify, up to 16 scores each.  Rows this cannot resolve (NaN, constant rows, massive
 // ties) fall back to the one-CTA selection.  The scores stay in L2 between the two readings.
 constexpr int kGroups = 8;
 constexpr int kGroupElems = 8;      // scores of qualifying groups a thread can hold
@@ -867,16 +869,34 @@ topk_pages_groups_kernel(const float *__restrict__ scores, PageOut page_list, in
     __syncthreads();
     if (warp == 0) descending_crossing(count_of, k, lane, &sh_digit, &sh_above, &sh_count, above_of);
     __syncthreads();
-    const int m = above_of[b1] + count_of[b1];   // every candidate: no bucket below b1 has any
+    // The bucket of the k-th score: what lies below it is left out.  If the buckets down to it still hold too many, it is
+    // split into 256 as the groups' were.
+    const int bk = sh_digit, above_k = sh_above;
+    int m = above_k + sh_count, split = 0;
+    const float lo_k = lo + (float)bk / lin_scale, scale_k = lin_scale * 256.f;
     if (m > cap) {
+        if (tid < 256) hist[1][tid] = 0;
         __syncthreads();
-        topk_row_fallback(srow, n_pages, k, dst, smem_raw);
-        return;
+#pragma unroll
+        for (int i = 0; i < kGroupElems; ++i)
+            if (id[i] >= 0 && linear_bucket(x[i], lo, lin_scale) == bk) atomicAdd(&hist[1][linear_bucket(x[i], lo_k, scale_k)], 1);
+        __syncthreads();
+        if (warp == 0) descending_crossing(hist[1], k - above_k, lane, &sh_digit, &sh_above, &sh_count);
+        __syncthreads();
+        split = sh_digit;
+        m = above_k + sh_above + sh_count;
+        if (m > cap) {
+            __syncthreads();
+            topk_row_fallback(srow, n_pages, k, dst, smem_raw);
+            return;
+        }
+        if (tid == 0) count_of[bk] = m - above_k;   // (read again behind the next barrier)
     }
 #pragma unroll
     for (int i = 0; i < kGroupElems; ++i) {
         if (id[i] < 0) continue;
         const int b = linear_bucket(x[i], lo, lin_scale);
+        if (b < bk || (b == bk && split > 0 && linear_bucket(x[i], lo_k, scale_k) < split)) continue;
         cand[above_of[b] + atomicAdd(&fill[b], 1)] =
             ((unsigned long long)(~score_key(x[i])) << 32) | (uint32_t)id[i];
     }

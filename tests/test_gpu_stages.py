@@ -808,7 +808,7 @@ def test_build_pages_bytes(da, hk, tokens, page, d, dtype, offset, extra):
 @pytest.mark.parametrize("pages,k", [(16385, 1), (16388, 1365), (16388, 1366), (32768, 300), (32769, 300), (32772, 682), (32772, 683),
                                      (65535, 256), (65536, 682), (65537, 200), (65540, 341), (65540, 342), (131072, 100),
                                      (131075, 256)])
-@pytest.mark.parametrize("kind", ["normal", "needles", "quantised", "outlier", "nan", "inf", "falling"])
+@pytest.mark.parametrize("kind", ["normal", "needles", "quantised", "outlier", "nan", "inf", "falling", "runs", "runs+needles"])
 def test_topk_long_rows_by_group_maxima(da, pages, k, kind):
     """Selection with one SM to count on, at both sides of every size at which the number of scores per group changes
     or the group path ends, against a stable descending sort of the same order (NaN above everything)."""
@@ -827,12 +827,43 @@ def test_topk_long_rows_by_group_maxima(da, pages, k, kind):
         sc[0, 3], sc[1, pages - 1] = float("inf"), float("-inf")
     elif kind == "falling":
         sc = sc.sort(-1, descending=True).values                     # the best scores side by side
+    if kind.startswith("runs"):                                      # neighbouring pages score alike
+        sc = torch.nn.functional.avg_pool1d(torch.randn(2, 1, pages + 24, generator=g) * 150, 25, stride=1)[:, 0]
+    if kind == "runs+needles":                                       # ... and most of the row is in a few buckets
+        sc[:, 1000:1000 + min(32, max(1, k // 2))] += 2000.0
     dev = sc.to(DEV)
     out = torch.full((1, 2 * k), -7, dtype=torch.int32, device=DEV)
     _native.check(_native.lib().da_topk_pages_wide(dev.data_ptr(), out.data_ptr(), 1, 1, 2, pages, k, 1,
                                                    _native.stream_ptr()))
     want = torch.sort(sc, dim=-1, descending=True, stable=True).indices[:, :k].reshape(1, -1).to(torch.int32)
     assert torch.equal(out.cpu(), want)
+
+
+@pytest.mark.parametrize("pages,k", [(20000, 256), (65536, 64), (65536, 512), (131072, 256)])
+def test_topk_time_does_not_depend_on_the_order_of_a_long_row(da, pages, k):
+    """The same scores shuffled, in runs of neighbours that score alike, and sorted: no order may leave the kernel's one
+    reading and a bit for the sweeps of the one-CTA selection, which take four times as long."""
+    from dram_attention_b200 import _native
+    base = torch.nn.functional.avg_pool1d(torch.randn(32, 1, pages + 24, generator=_g(k)) * 150, 25, stride=1)[:, 0]
+    out = torch.empty(8, 4 * k, dtype=torch.int32, device=DEV)
+
+    def us(rows):
+        dev = rows.contiguous().to(DEV)
+        best = float("inf")
+        for _ in range(6):      # the first one warms up
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(20):
+                _native.check(_native.lib().da_topk_pages(dev.data_ptr(), out.data_ptr(), 1, 8, 4, pages, k,
+                                                          _native.stream_ptr()))
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 50)
+        return best
+
+    shuffled = us(base[:, torch.randperm(pages, generator=_g(pages))])
+    for rows in (base, base.sort(-1, descending=True).values):
+        assert us(rows) <= 2 * shuffled
 
 
 @pytest.mark.parametrize("pages,k,s", [(100, 8, 3), (5000, 300, 2), (12000, 64, 1), (40000, 200, 2), (65536, 1500, 1)])
