@@ -2,12 +2,13 @@
 // code.  Enqueued one by one from an interpreted caller the launches, stream switches and events of a step took
 // about 110 us of host time, three times what the GPU needs for them.
 
+#include <new>
+
 #include "da_common.cuh"
 
 namespace da {
 
 struct Fork {
-    int device;
     cudaStream_t side;
     cudaEvent_t started, joined;
 };
@@ -67,9 +68,9 @@ static int update_tables(const da_generate_args &a, int advance, bool inline_fet
 
 extern "C" int da_fork_create(void **fork) {
     if (!fork) return DA_ERR_NULL;
-    da::Fork *f = new da::Fork();
-    cudaError_t e = cudaGetDevice(&f->device);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&f->side, cudaStreamNonBlocking);
+    da::Fork *f = new (std::nothrow) da::Fork();
+    if (!f) return (int)cudaErrorMemoryAllocation;
+    cudaError_t e = cudaStreamCreateWithFlags(&f->side, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&f->started, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&f->joined, cudaEventDisableTiming);
     if (e != cudaSuccess) {
@@ -126,10 +127,16 @@ extern "C" int da_generate(const da_generate_args *args) {
     if (!early && (e = cudaEventRecord(f->started, main)) != cudaSuccess) return (int)e;
     if ((rc = da::select_pages(a, budget)) != 0) return rc;
     if ((e = cudaStreamWaitEvent(f->side, f->started, 0)) != cudaSuccess) return (int)e;
-    if ((rc = da::attention_phase(a, 1, f->side)) != 0) return rc;
-    if ((e = cudaEventRecord(f->joined, f->side)) != cudaSuccess) return (int)e;
-    if ((rc = da::update_tables(a, 2, true)) != 0) return rc;
+    const int rc1 = da::attention_phase(a, 1, f->side);
+    rc = rc1;
+    if (rc == 0) rc = da::update_tables(a, 2, true);
     // phase 2 needs the update, not phase 1: whichever of the two launches finishes last merges
-    if ((rc = da::attention_phase(a, 2, main)) != 0) return rc;
-    return (int)cudaStreamWaitEvent(main, f->joined, 0);
+    if (rc == 0) rc = da::attention_phase(a, 2, main);
+    // The fork's stream is joined whatever became of the launches: phase 1 reads the caller's tensors, and a capture ends
+    // only with all its streams joined.
+    if ((e = cudaEventRecord(f->joined, f->side)) == cudaSuccess) e = cudaStreamWaitEvent(main, f->joined, 0);
+    // Phase 1 without its phase 2 leaves its tickets in the workspace, which the next call would count as its own.
+    if (rc != 0 && rc1 == 0 && e == cudaSuccess)
+        e = cudaMemsetAsync(a.workspace, 0, (size_t)a.n_kv_heads * sizeof(unsigned int), main);
+    return rc != 0 ? rc : (int)e;
 }

@@ -566,7 +566,8 @@ DA_API int da_gather_heads(const void *local, int bytes_per_rank, void *const *p
  *   selection_sm_budget   0: 148 minus phase 1's CTAs
  *   peer_buffers (may be null), peer_seq, peer_rank, peer_world, peer_bytes   as da_decode_attention_push_next
  * Scores, page list and the miss list are scratch of the caller, sized for n_q_tokens.  The call works inside a stream
- * capture.  The fork's stream is joined to `stream` before the call returns.
+ * capture.  The fork's stream is joined to `stream` before the call returns,
+ * also when it returns an error; a step that failed half-way leaves the ticket words of the workspace zero.
  */
 #define DA_LAYOUT_RESIDENT 0
 #define DA_LAYOUT_FETCH_KERNEL 1

@@ -821,3 +821,40 @@ def test_two_launch_step_repeats_bit_for_bit(da, hk, rep, d, dtype):
         outs.append(out.clone())
     assert all(torch.equal(outs[0], o) for o in outs[1:])
     m.check_status()
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_a_step_that_fails_half_way_leaves_nothing_behind(da, captured):
+    """The update of a two-launch step is refused (its status word is missing) when phase 1 is on its way already: the call
+    raises, the side stream is joined (a capture can end), and the following steps, in either layout, are those of a
+    twin that never failed."""
+    (m, twin), x, pos = _two_launch_operators(da, 2, 2, 4, 128, torch.bfloat16, 3, False)
+    lc = m.lru_cache
+    status = lc.status
+
+    def fail():
+        lc.status = torch.empty(0, dtype=torch.int32, device=DEV)
+        try:
+            with pytest.raises(RuntimeError, match="da_generate"):
+                m(*x, start_pos=pos, stage="generate")
+        finally:
+            lc.status = status
+
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):
+            fail()
+        graph.replay()
+    else:
+        fail()
+    torch.cuda.synchronize()
+    assert all(not bool(w[0][:1024].any()) for w in m._ws.values())
+    for i, overlap in enumerate((True, False, True)):
+        m.overlap = twin.overlap = overlap
+        a, b = (op(*x, start_pos=pos + i, stage="generate") for op in (m, twin))
+        assert torch.equal(a, b)
+    assert torch.equal(m.lru_cache.hbm_page_to_dram_page_mapping, twin.lru_cache.hbm_page_to_dram_page_mapping)
+    assert torch.equal(m.cache_k, twin.cache_k)
+    for op in (m, twin):
+        op.check_status()
