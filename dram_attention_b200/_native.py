@@ -5,6 +5,7 @@ the import of any operator fails with instructions to build it."""
 from __future__ import annotations
 
 import ctypes
+import operator
 import os
 import struct
 from ctypes import c_char_p, c_float, c_int, c_int32, c_longlong, c_size_t, c_void_p, POINTER
@@ -131,6 +132,18 @@ class Fork:
         if self.handle:
             self._destroy(self.handle)
             self.handle = None
+
+
+def own_methods(cls: type, *names: str):
+    """A check whether an object's methods of the given names are still those that `cls` has now: neither
+    overridden by a subclass, nor replaced in the class or in the instance."""
+    get = operator.attrgetter(*names)
+    methods, names = get(cls), frozenset(names)
+
+    def own(obj) -> bool:
+        return isinstance(obj, cls) and get(type(obj)) == methods and obj.__dict__.keys().isdisjoint(names)
+
+    return own
 
 
 def check(code: int, what: str = "") -> None:

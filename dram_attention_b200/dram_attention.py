@@ -266,7 +266,8 @@ class DRAMAttention(torch.nn.Module):
             layout = _native.LAYOUT_OVERLAPPED
         else:
             layout = _native.LAYOUT_FETCH_IN_ATTENTION
-        if layout != _native.LAYOUT_RESIDENT and not lc.updates_natively():
+        if not (_own_stages(self) and (_own_dummy_stages(lc) if layout == _native.LAYOUT_RESIDENT
+                                       else isinstance(lc, LRUCache) and lc.updates_natively())):
             self._generate_stage_by_stage(layout, xq, xk, xv, start_pos, out)
             return out
         if isinstance(start_pos, torch.Tensor):
@@ -304,7 +305,8 @@ class DRAMAttention(torch.nn.Module):
         return out
 
     def _generate_stage_by_stage(self, layout: int, xq, xk, xv, start_pos, out) -> None:
-        """The same launches through the classes' own methods, for a cache whose update_tables_ was replaced."""
+        """The same launches through the methods of the operator, its cache and its selector, each of which may have been
+        overridden or replaced."""
         lc = self.lru_cache
         if layout == _native.LAYOUT_OVERLAPPED:
             self._generate_overlapped(xq, xk, xv, start_pos, out)
@@ -427,3 +429,8 @@ class DRAMAttention(torch.nn.Module):
                 raise RuntimeError("dram_attention_b200 device status: " + _native.status_message(bits))
         if isinstance(self.lru_cache, LRUCache):
             self.lru_cache.check_status()
+
+
+# what a generate call goes through, stage by stage
+_own_stages = _native.own_methods(DRAMAttention, "attend_", "_generate_overlapped")
+_own_dummy_stages = _native.own_methods(DummyCache, "get_kv_cache_", "kv_views")

@@ -230,9 +230,9 @@ class LRUCache(torch.nn.Module):
             self.status.data_ptr(), _native.stream_ptr()), "da_lru_update")
 
     def updates_natively(self) -> bool:
-        """Whether a generate call may enqueue the update itself instead of calling update_tables_ (it may not
-        when a subclass or the instance replaced that method)."""
-        return type(self).update_tables_ is LRUCache.update_tables_ and "update_tables_" not in self.__dict__
+        """Whether a generate call may enqueue selection, update and fetch itself instead of calling this cache's and
+        its selector's methods (it may not when a subclass or the instance replaced one of them)."""
+        return _own_cache_stages(self) and _own_selector_stages(self.top_k_selector)
 
     NO_GENERATE_FIELDS = (0,) * 23
 
@@ -305,3 +305,8 @@ class LRUCache(torch.nn.Module):
         if bits:
             self.status.zero_()
             raise RuntimeError("dram_attention_b200 device status: " + _native.status_message(bits))
+
+
+# what a generate call goes through, stage by stage
+_own_cache_stages = _native.own_methods(LRUCache, "get_kv_cache_", "_load_int32_", "update_tables_", "fetch_")
+_own_selector_stages = _native.own_methods(IPUpperboundTopKSelector, "page_list_", "score_", "select_")

@@ -740,7 +740,7 @@ def _two_launch_operators(da, n, hk, rep, d, dtype, steps, redraw):
     length, page = 6000, 16
     k, v = (torch.randn(1, length, hk, d, generator=g).to(dtype).to(DEV) for _ in range(2))
     u = torch.randn(hk * rep, d, generator=g)
-    ms = [da.DRAMAttention(max_output_length=steps + 4, lru_hbm_cache_size=1536, local_cache_size=300, page_size=page,
+    ms = [da.DRAMAttention(max_output_length=steps + 16, lru_hbm_cache_size=1536, local_cache_size=300, page_size=page,
                            top_k=page * max(1, 60 // rep), n_kv_heads=hk, head_dim=d, device=DEV, dtype=dtype)
           for _ in range(n)]
     for m in ms:
@@ -858,3 +858,43 @@ def test_a_step_that_fails_half_way_leaves_nothing_behind(da, captured):
     assert torch.equal(m.cache_k, twin.cache_k)
     for op in (m, twin):
         op.check_status()
+
+
+@pytest.mark.parametrize("layout,tokens,stages", [
+    ((True, True), 1, {"sel": ["score_", "select_"], "lc": ["update_tables_"], "op": ["attend_", "_generate_overlapped"]}),
+    ((True, False), 1, {"sel": ["score_", "select_", "page_list_"], "lc": ["update_tables_"], "op": ["attend_"]}),
+    ((False, False), 1, {"sel": ["score_", "select_", "page_list_"], "op": ["attend_"],
+                         "lc": ["get_kv_cache_", "_load_int32_", "update_tables_", "fetch_"]}),
+    ((True, True), 2, {"sel": ["page_list_"], "lc": ["get_kv_cache_", "fetch_"], "op": ["attend_"]}),
+], ids=["overlapped", "fetch-in-attention", "fetch-kernel", "two-tokens"])
+def test_a_replaced_stage_is_called(da, layout, tokens, stages):
+    """Whichever stage of a generate call a program wraps (to trace it, or to put its own in), the call goes through it,
+    with the result of an untouched operator."""
+    (m, twin), x, pos = _two_launch_operators(da, 2, 2, 4, 128, torch.bfloat16, 2, False)
+    x = [t.expand(1, tokens, -1, -1).contiguous() for t in x]
+    for op in (m, twin):
+        op.fused_fetch, op.overlap = layout
+    for owner, names in stages.items():
+        for name in names:
+            obj = {"sel": m.lru_cache.top_k_selector, "lc": m.lru_cache, "op": m}[owner]
+            calls, own = [], getattr(obj, name)
+            obj.__dict__[name] = lambda *a, _own=own, _calls=calls, **k: (_calls.append(1), _own(*a, **k))[1]
+            a = m(*x, start_pos=pos, stage="generate")
+            del obj.__dict__[name]
+            assert calls, (owner, name)
+            assert torch.equal(a, twin(*x, start_pos=pos, stage="generate")), (owner, name)
+            pos += tokens
+    assert torch.equal(m.lru_cache.hbm_kv_cache, twin.lru_cache.hbm_kv_cache)
+
+
+def test_a_replaced_resident_cache_is_called(da):
+    g = torch.Generator().manual_seed(1)
+    k, v = (torch.randn(1, 900, 2, 128, generator=g).to(torch.bfloat16).to(DEV) for _ in range(2))
+    m = da.DRAMAttention(max_output_length=4, lru_hbm_cache_size=1024, local_cache_size=200, page_size=16, top_k=256,
+                         n_kv_heads=2, head_dim=128, device=DEV)
+    m.init_cache(k, v)
+    x = [torch.randn(1, 1, h, 128, generator=g).to(torch.bfloat16).to(DEV) for h in (8, 2, 2)]
+    want = m(*x, start_pos=900, stage="generate")
+    calls, own = [], m.lru_cache.get_kv_cache_
+    m.lru_cache.get_kv_cache_ = lambda q: (calls.append(q.shape), own(q))[1]
+    assert torch.equal(m(*x, start_pos=900, stage="generate"), want) and calls == [x[0].shape]
