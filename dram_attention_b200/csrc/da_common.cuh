@@ -141,33 +141,63 @@ cudaError_t trace_set_gather(void *buffer);
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// The launches of that chain go ahead of work of the default priority when an SM falls free: the first attention launch
-// of another sequence on another stream takes whole SMs, as the selection does, and kept it waiting for 60 us.  Eight
-// sequences of 64K on four streams: 301 -> 291 us (with the scorer too: 296); a single sequence is unchanged.
-constexpr int kChainPriority = -1;
+// The dependent launches of a two-launch step (selection, update, phase 2) go ahead of work of the priority their stream has when
+// an SM falls free: the first attention launch of another sequence on another stream takes whole SMs, as the selection
+// does, and kept it waiting for 60 us.  Eight sequences of 64K on four streams: 301 -> 291 us (with the scorer too: 296); a
+// single sequence is unchanged.  Every other launch has its stream's priority, so calls that only select, update or attend
+// do not overtake the rest of the program.
+// While one lives, launch_dependent() of this thread launches one level above the priority of `stream` (none for a stream
+// that has the highest already).
+inline thread_local int ahead_priority = 0;   // 0: the stream's own
+struct AheadOfStream {
+    explicit AheadOfStream(cudaStream_t stream) {
+        static const int greatest = [] {   // (the same for every device of one kind)
+            int least = 0, most = 0;
+            if (cudaDeviceGetStreamPriorityRange(&least, &most) == cudaSuccess) return most;
+            (void)cudaGetLastError();
+            return 0;
+        }();
+        int own = 0;      // that of the default stream
+        if (stream != nullptr && cudaStreamGetPriority(stream, &own) != cudaSuccess) (void)cudaGetLastError();   // (the launches will say why)
+        else if (own > greatest) ahead_priority = own - 1;
+    }
+    ~AheadOfStream() { ahead_priority = 0; }
+    AheadOfStream(const AheadOfStream &) = delete;
+    AheadOfStream &operator=(const AheadOfStream &) = delete;
+};
 
+// `cluster`: CTAs per cluster (1: none).
 template <typename... KArgs, typename... Args>
-static inline cudaError_t launch_dependent_at(int priority, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                              cudaStream_t stream, Args... args) {
+static inline cudaError_t launch_dependent_clusters(int cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                                    cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributePriority;
-    attr[1].val.priority = priority;
+    cudaLaunchAttribute attr[3];
+    unsigned n = 0;
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    if (ahead_priority != 0) {
+        attr[n].id = cudaLaunchAttributePriority;
+        attr[n++].val.priority = ahead_priority;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = priority != 0 ? 2 : 1;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
 template <typename... KArgs, typename... Args>
 static inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                            cudaStream_t stream, Args... args) {
-    return launch_dependent_at(0, kernel, grid, block, smem, stream, args...);
+    return launch_dependent_clusters(1, kernel, grid, block, smem, stream, args...);
 }
 
 // The scorer behind da_score_pages; `started` (may be null) is recorded when all its CTAs have begun.

@@ -668,14 +668,14 @@ static cudaError_t launch_lru(const LruArgs &a, cudaStream_t stream) {
     }
     if (a.queue) {
         const size_t tables = lru_queue_smem_bytes(a.n_slots, a.list_len);
-        return launch_dependent_at(kChainPriority, lru_queue_kernel<SR, LR>, dim3(a.n_kv_heads), dim3(kLruThreads),
+        return launch_dependent(lru_queue_kernel<SR, LR>, dim3(a.n_kv_heads), dim3(kLruThreads),
                                 tables + (size_t)a.inline_max * a.page_bytes, stream, a.page_list, a.list_len,
                                 a.dram_to_slot, a.n_dram_pages, a.slot_to_dram, a.access_time, a.n_slots, a.step,
                                 a.miss_pages, a.miss_slots, a.n_miss, a.slot_source, a.queue, a.n_front,
                                 a.split_flip, a.split_redo, a.split_cap, a.split_advance, a.dram_pages, a.slots,
                                 a.page_bytes, a.inline_max, (unsigned int)tables, a.status);
     }
-    return launch_dependent_at(kChainPriority, lru_update_kernel<SR, LR>, dim3(a.n_kv_heads), dim3(kLruThreads),
+    return launch_dependent(lru_update_kernel<SR, LR>, dim3(a.n_kv_heads), dim3(kLruThreads),
                             lru_smem_bytes(a.n_slots, a.list_len), stream, a.page_list, a.list_len,
                             a.dram_to_slot, a.n_dram_pages, a.slot_to_dram, a.access_time, a.n_slots, a.step,
                             a.miss_pages, a.miss_slots, a.n_miss, a.slot_source, a.status);

@@ -125,6 +125,7 @@ extern "C" int da_generate(const da_generate_args *args) {
         if (budget < 1) budget = 1;
     }
     if (!early && (e = cudaEventRecord(f->started, main)) != cudaSuccess) return (int)e;
+    const da::AheadOfStream ahead(main);   // selection, update and phase 2
     if ((rc = da::select_pages(a, budget)) != 0) return rc;
     if ((e = cudaStreamWaitEvent(f->side, f->started, 0)) != cudaSuccess) return (int)e;
     const int rc1 = da::attention_phase(a, 1, f->side);

@@ -929,7 +929,7 @@ static cudaError_t launch_topk(const float *scores, PageOut page_list, int rows,
     }
     const int cap = topk_candidate_capacity(k);
     const size_t smem = (size_t)(cap + 2) * sizeof(unsigned long long) + (size_t)cap * sizeof(int);
-    const cudaError_t le = launch_dependent_at(kChainPriority, topk_pages_kernel<IPT>, dim3(rows), dim3(kTopkThreads), (size_t)smem, stream,
+    const cudaError_t le = launch_dependent(topk_pages_kernel<IPT>, dim3(rows), dim3(kTopkThreads), (size_t)smem, stream,
                                             scores, page_list, n_kv_heads, rep, n_pages, k);
     if (le != cudaSuccess) return le;
     return cudaGetLastError();
@@ -940,7 +940,7 @@ static cudaError_t launch_topk_groups(const float *scores, PageOut page_list, in
                                       int n_pages, int k, cudaStream_t stream) {
     const int cap = topk_candidate_capacity(k);      // at most 2048 here: 24 KB, no opt-in needed
     const size_t smem = (size_t)(cap + 2) * sizeof(unsigned long long) + (size_t)cap * sizeof(int);
-    const cudaError_t e = launch_dependent_at(kChainPriority, topk_pages_groups_kernel<PER, VEC>, dim3(rows), dim3(kTopkThreads), smem, stream,
+    const cudaError_t e = launch_dependent(topk_pages_groups_kernel<PER, VEC>, dim3(rows), dim3(kTopkThreads), smem, stream,
                                            scores, page_list, n_kv_heads, rep, n_pages, k);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -967,21 +967,9 @@ static cudaError_t launch_topk_cluster(const float *scores, PageOut page_list, i
         attr_set[dev] = true;
     }
     const int cap = topk_candidate_capacity(k);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(rows * kTopkCluster);
-    cfg.blockDim = dim3(kTopkThreads);
-    cfg.dynamicSmemBytes = (size_t)(cap + 2) * sizeof(unsigned long long) + (size_t)cap * sizeof(int);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = kTopkCluster;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
-    e = cudaLaunchKernelEx(&cfg, topk_pages_cluster_kernel, scores, page_list, n_kv_heads, rep, n_pages, k);
+    const size_t smem = (size_t)(cap + 2) * sizeof(unsigned long long) + (size_t)cap * sizeof(int);
+    e = launch_dependent_clusters(kTopkCluster, topk_pages_cluster_kernel, dim3(rows * kTopkCluster), dim3(kTopkThreads), smem,
+                                  stream, scores, page_list, n_kv_heads, rep, n_pages, k);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }

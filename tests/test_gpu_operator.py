@@ -898,3 +898,62 @@ def test_a_replaced_resident_cache_is_called(da):
     calls, own = [], m.lru_cache.get_kv_cache_
     m.lru_cache.get_kv_cache_ = lambda q: (calls.append(q.shape), own(q))[1]
     assert torch.equal(m(*x, start_pos=900, stage="generate"), want) and calls == [x[0].shape]
+
+
+def _captured_kernel_priorities(call, stream):
+    """Priorities of the kernels a call enqueues on `stream`, in the graph it is captured into."""
+    runtime = pytest.importorskip("cuda.bindings.runtime")
+    ok = runtime.cudaError_t.cudaSuccess
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+    raw = runtime.cudaGraph_t(graph.raw_cuda_graph())
+    err, _, n = runtime.cudaGraphGetNodes(raw)
+    assert err == ok
+    err, nodes, n = runtime.cudaGraphGetNodes(raw, n)
+    assert err == ok
+    found = []
+    for node in nodes[:n]:
+        err, kind = runtime.cudaGraphNodeGetType(node)
+        assert err == ok
+        if kind == runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel:
+            err, value = runtime.cudaGraphKernelNodeGetAttribute(node, runtime.cudaLaunchAttributeID.cudaLaunchAttributePriority)
+            assert err == ok
+            found.append(value.priority)
+    return sorted(found)
+
+
+@pytest.mark.parametrize("own", [0, -2])
+def test_only_the_chain_of_a_two_launch_step_goes_ahead(da, own):
+    """Selection, update and phase 2 of a two-launch step are one priority level above the caller's stream, phase 1 on the
+    side stream at the lowest; everything else (the scorer, other layouts, a bare selection or load) runs at the stream's."""
+    stream = torch.cuda.Stream(priority=own)
+    (m,), x, pos = _two_launch_operators(da, 1, 2, 4, 128, torch.bfloat16, 2, False)
+    step = lambda: m(*x, start_pos=pos, stage="generate")
+    lc = m.lru_cache
+    lc.top_k_selector.top_k(x[0], lc.top_k)                                   # (allocations and first launches)
+    ids = torch.arange(8, device=DEV, dtype=torch.int32).repeat(2, 1)
+    lc.load_(ids)
+    assert _captured_kernel_priorities(step, stream) == sorted([own, own - 1, own - 1, own - 1, 0])
+    for layout, n in (((True, False), 4), ((False, False), 5)):
+        m.fused_fetch, m.overlap = layout
+        step()
+        assert _captured_kernel_priorities(step, stream) == [own] * n
+    assert _captured_kernel_priorities(lambda: lc.top_k_selector.top_k(x[0], lc.top_k), stream) == [own] * 2
+    assert _captured_kernel_priorities(lambda: lc.load_(ids), stream) == [own] * 2
+
+
+def test_a_long_row_cluster_of_the_chain_goes_ahead(da):
+    """The same where a large k takes the selection to clusters."""
+    g = torch.Generator().manual_seed(2)
+    k = torch.randn(1, 17000, 1, 64, generator=g).to(torch.bfloat16).to(DEV).repeat_interleave(16, 1)
+    m = da.DRAMAttention(max_output_length=4, lru_hbm_cache_size=4096 * 16, local_cache_size=64, page_size=16,
+                         top_k=2000 * 16, n_kv_heads=1, head_dim=64, device=DEV)
+    m.init_cache(k, k)
+    x = [torch.randn(1, 1, 1, 64, generator=g).to(torch.bfloat16).to(DEV) for _ in range(3)]
+    step = lambda: m(*x, start_pos=k.shape[1], stage="generate")
+    step()
+    assert m.lru_cache.num_dram_pages > 16384
+    assert _captured_kernel_priorities(step, torch.cuda.Stream()) == [-1, -1, -1, 0, 0]
+    m.check_status()
