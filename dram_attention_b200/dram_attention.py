@@ -75,7 +75,8 @@ class DRAMAttention(torch.nn.Module):
     # ... and that first launch starts once every CTA of the page scorer has begun, taking over the SMs as they
     # leave them, rather than after the scorer.  (Waiting for the scorer's start, not merely being enqueued
     # behind it, is what keeps a graph from dispatching it first: it then left the scorer 32 of 148 SMs and a
-    # 128K layer took 60 us instead of 40.)
+    # 128K layer took 60 us instead of 40.)  A call that goes stage by stage, because a method of it was replaced,
+    # always starts it after the scorer.
     fork_before_score = True
     # CTAs per KV head of the two launches (0: the library's defaults)
     phase1_ctas = 0
@@ -328,7 +329,7 @@ class DRAMAttention(torch.nn.Module):
         return ok
 
     def _generate_overlapped(self, xq, xk, xv, start_pos, out) -> None:
-        """{ score -> select -> LRU update -> attention phase 2 }  ||  attention phase 1."""
+        """{ score -> select -> LRU update -> attention phase 2 }  ||  attention phase 1, through the methods."""
         lc = self.lru_cache
         sel = lc.top_k_selector
         rep = xq.shape[2] // self.n_kv_heads
@@ -336,28 +337,19 @@ class DRAMAttention(torch.nn.Module):
             self._side = torch.cuda.Stream(device=xq.device)
             self._fork, self._join = torch.cuda.Event(), torch.cuda.Event()
         main = torch.cuda.current_stream()
-        # Phase 1 needs nothing this step computes (only the split the previous step left), so it
-        # forks off before the scorer: its CTAs move onto the SMs as the scorer's short CTAs leave
-        # them.  The scorer is launched first so that the chain score -> select -> update is not
-        # the one that waits for SMs.
-        # Only inside a graph capture: a graph dispatches the scorer's CTAs ahead of phase 1's (node
-        # order), whereas two eager launches that become ready together (a backlogged GPU) may be
-        # dispatched either way round, and phase 1 first would starve the scorer of SMs.
+        # Phase 1 needs nothing this step computes (only the split the previous step left).  Here it forks off after the
+        # scorer: an event in front of the scorer says nothing about which of the two gets the SMs first, and phase 1
+        # first leaves the scorer 32 of them (four captured 128K layers: 186 us, forked after the scorer 174).  Between the
+        # two lies the start of the scorer's last CTA, which only the library call waits for (164).
         budget = self.selection_sm_budget or max(1, 148 - self.n_kv_heads * (
             self.phase1_ctas or _native.lib().da_decode_attention_phase1_ctas(self.n_kv_heads)))
-        early = self.fork_before_score and torch.cuda.is_current_stream_capturing()
-        if early:
-            self._fork.record(main)
         sel.score_(xq, lc.top_k)
-        if not early:
-            self._fork.record(main)
-            page_list = sel.select_(1, rep, lc.top_k, sm_budget=budget)     # ahead of phase 1, so that its CTAs find SMs free
+        self._fork.record(main)
+        page_list = sel.select_(1, rep, lc.top_k, sm_budget=budget)     # ahead of phase 1, so that its CTAs find SMs free
         self._side.wait_event(self._fork)
         with torch.cuda.stream(self._side):
             self.attend_(xq, xk, xv, start_pos, out, phase=1)
             self._join.record(self._side)
-        if early:
-            page_list = sel.select_(1, rep, lc.top_k, sm_budget=budget)
         lc.update_tables_(page_list, advance_split=False, inline_fetch=True, after_selection=True)
         # phase 2 needs the update, not phase 1: whichever of the two launches finishes last merges
         self.attend_(xq, xk, xv, start_pos, out, phase=2)
