@@ -313,22 +313,24 @@ static int run_attention(const AttnCall &c) {
 
     // the single launch: at least two units per warp, so that a short prefix does not pay for merging empty rows
     int splits0 = attn_splits(c.n_kv_heads);
-    const int unit_splits = (c.n_prefix_tokens + c.local_capacity) / (2 * kUnitTokens * kAttnWarps) + 1;
-    if (splits0 > unit_splits) splits0 = unit_splits;
+    const long long unit_splits = ((long long)c.n_prefix_tokens + c.local_capacity) / (2 * kUnitTokens * kAttnWarps) + 1;
+    if (splits0 > unit_splits) splits0 = (int)unit_splits;
     const int ctas = c.phase == 0 ? splits0 : c.splits1 + c.splits2;
     // Query tokens per launch.  More than 16 rows (16-bit types) go 32 at a time, so that the keys and values are
     // read half as often, where the workspace has room for so many rows (with one KV head it has not).  us for five
     // tokens of rep 4 over 36 900 slot and window tokens x 8 heads: two launches 64, one 47.
     int tokens_per_launch = max_rows_of(c.dtype) / c.rep;
     auto rows_of = [&](int per_launch) { return (c.n_q_tokens < per_launch ? c.n_q_tokens : per_launch) * c.rep; };
+    // the workspace has its stated size, whatever part of it this launch touches
+    const int stated = c.phase == 0 ? attn_reserved_splits(c.n_kv_heads) : ctas;
+    if (c.workspace_bytes < (size_t)kCounterBytes + partial_bytes(c.n_kv_heads, stated, rows_of(tokens_per_launch), c.head_dim))
+        return DA_ERR_WORKSPACE;
     if (c.dtype != DA_F32 && c.n_q_tokens > tokens_per_launch) {
         const int wide = kAttnWideRows / c.rep;
         if (c.workspace_bytes >= (size_t)kCounterBytes + partial_bytes(c.n_kv_heads, ctas, rows_of(wide), c.head_dim))
             tokens_per_launch = wide;
     }
     const int rows_max = rows_of(tokens_per_launch);
-    if (c.workspace_bytes < (size_t)kCounterBytes + partial_bytes(c.n_kv_heads, ctas, rows_max, c.head_dim))
-        return DA_ERR_WORKSPACE;
     // phase 1's partials merged into one, where the workspace (the same one for both launches) has room for one more
     const size_t one_more = (size_t)kCounterBytes + partial_bytes(c.n_kv_heads, ctas + 1, rows_max, c.head_dim);
     const int part_rows = ctas + (c.phase != 0 && c.workspace_bytes >= one_more ? 1 : 0);

@@ -77,6 +77,11 @@ def test_host_side_argument_checks(native):
     assert lib.da_decode_attention(*bad) == -4                                # alignment
     bad = list(args); bad[17] = 16
     assert lib.da_decode_attention(*bad) == -6                                # workspace
+    for tokens, dtype in ((1, 2), (3, 2), (9, 1), (1, 0), (5, 0)):             # one byte less than stated, short prefix or long
+        need = lib.da_decode_attention_tokens_workspace_bytes(8, 4, 128, tokens if dtype else min(tokens, 2))
+        for prefix in (16, 1 << 20, 0x7fffffff):
+            assert lib.da_decode_attention_tokens(256, tokens, 256, 4096, prefix, 256, 256, 1024, 128, 64, 256, 256, 0, 0,
+                                                  0, 256, 0, 256, need - 1, 256, 8, 4, 128, dtype, 0) == -6
     bad = list(args); bad[22] = 9
     assert lib.da_decode_attention(*bad) == -3                                # dtype
     bad = list(args); bad[20] = 17
