@@ -125,8 +125,8 @@ class Fork:
         check(lib().da_fork_create(ctypes.byref(out)), "da_fork_create")
         self.handle, self._destroy = out.value, lib().da_fork_destroy
 
-    def __deepcopy__(self, memo):
-        return Fork()
+    def __reduce__(self):
+        return type(None), ()   # a copied or saved operator makes one of its own, on its device, when it needs it
 
     def __del__(self):
         if self.handle:

@@ -1,5 +1,8 @@
 """A generate call is enqueued as one library call only while every stage method is the package's own."""
 
+import copy
+import pickle
+
 import pytest
 
 from dram_attention_b200 import DRAMAttention, _native
@@ -44,3 +47,10 @@ def test_a_cache_asks_for_its_selector_too():
     assert not cache.updates_natively()
     cache.__dict__["top_k_selector"] = object()
     assert not cache.updates_natively()
+
+
+def test_a_fork_is_not_copied_or_saved():
+    fork = _bare(_native.Fork)
+    fork.handle, fork._destroy = None, _native.lib().da_fork_destroy
+    holder = {"_fork_handle": fork, "x": 1}
+    assert copy.deepcopy(holder) == pickle.loads(pickle.dumps(holder)) == {"_fork_handle": None, "x": 1}
