@@ -126,7 +126,7 @@ DA_API int da_topk_pages(const float *scores, int32_t *page_list,
 
 /*
  * The same selection with a hint on how many SMs it may count on.  Rows of 16 385 to 65 536
- * pages with a large k (above 682 to 1365, by their length) are split over a thread-block cluster of four CTAs (partial
+ * pages with a large k (above 1365, of more than 32 768 pages above 683) are split over a thread-block cluster of four CTAs (partial
  * histograms summed through distributed shared memory, candidates collected in one CTA) when all
  * clusters of the launch find an SM per CTA at once: n_tokens * n_kv_heads * rep * 4 <= sm_budget.  A caller
  * that runs another launch beside the selection (the first attention launch of the two-launch

@@ -26,29 +26,35 @@ def da():
     return pkg
 
 
-@pytest.fixture(params=[(True, True), (True, False), (False, False)],
-                ids=["overlapped", "fetch-in-attention", "fetch-kernel"])
-def fused(request, da):
+@pytest.fixture(params=[(True, True), (True, False), (False, False), "staged"],
+                ids=["overlapped", "fetch-in-attention", "fetch-kernel", "stage-by-stage"])
+def fused(request, da, monkeypatch):
     """The three ways a generate step can be laid out: two attention launches with the first
     beside selection and LRU update; one attention launch that also brings the missed pages in;
-    a gather-copy launch followed by the attention launch.  All give the same results."""
-    old = (da.DRAMAttention.fused_fetch, da.DRAMAttention.overlap)
-    da.DRAMAttention.fused_fetch, da.DRAMAttention.overlap = request.param
-    yield request.param
-    da.DRAMAttention.fused_fetch, da.DRAMAttention.overlap = old
+    a gather-copy launch followed by the attention launch.  All give the same results.  The fourth is the
+    first one as a program gets it that has replaced a method: every stage through its method."""
+    op = da.DRAMAttention
+    if request.param == "staged":
+        own = op._generate_overlapped
+        monkeypatch.setattr(op, "_generate_overlapped", lambda self, *args: own(self, *args))
+    else:
+        monkeypatch.setattr(op, "fused_fetch", request.param[0])
+        monkeypatch.setattr(op, "overlap", request.param[1])
+    return request.param
 
 
 def _spy_lists(module):
-    """Record the page list of every step (a copy of the selector's int32 output)."""
+    """Record the page list of every step: a copy of the selector's int32 output after the call.  Nothing is replaced, so
+    the call takes the way it takes in any program."""
     lists = []
-    lc = module.lru_cache
-    orig = lc.update_tables_
 
-    def spy(page_list, **kw):
-        lists.append(page_list.clone())
-        return orig(page_list, **kw)
+    def after(m, args, kwargs, output):
+        sel, seq_len = m.lru_cache.top_k_selector, args[0].shape[1]
+        rep = args[0].shape[2] // m.n_kv_heads
+        assert m.lru_cache.updates_natively()
+        lists.append(sel._buffers[(seq_len, rep, min(m.lru_cache.top_k, sel.num_pages))][1].clone())
 
-    lc.update_tables_ = spy
+    module.register_forward_hook(after, with_kwargs=True)
     return lists
 
 
@@ -453,21 +459,13 @@ def test_long_run_of_captured_steps_agrees_with_the_plain_layout(da):
     dq, dk, dv = w.xq.to(DEV), w.xk.to(DEV), w.xv.to(DEV)
     a(dq[0], dk[0], dv[0], start_pos=S, stage="generate")        # workspaces, side stream
     b(dq[0], dk[0], dv[0], start_pos=S, stage="generate")
-    rep = w.n_q_heads // w.n_kv_heads
+    lists = _spy_lists(a)      # (the copies are part of the graph)
     for first in range(1, n - k_graph + 1, k_graph):
-        lists = []
-        orig = a.lru_cache.update_tables_
-
-        def spy(page_list, **kw):
-            lists.append(page_list.clone())
-            return orig(page_list, **kw)
-
-        a.lru_cache.update_tables_ = spy
+        del lists[:]
         torch.cuda.synchronize()
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
             outs = [a(dq[i], dk[i], dv[i], start_pos=S + i, stage="generate") for i in range(first, first + k_graph)]
-        a.lru_cache.update_tables_ = orig
         g.replay()
         torch.cuda.synchronize()
         for j, i in enumerate(range(first, first + k_graph)):

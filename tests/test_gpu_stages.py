@@ -121,10 +121,17 @@ def _topk_oracle(scores, hk, rep, k):
     (300, 300, 2, 1, 1, "normal"), (4096, 4096, 1, 1, 1, "normal"), (1, 1, 2, 2, 1, "normal"),
     (8192, 256, 2, 4, 1, "quantised"), (3000, 500, 2, 2, 1, "quantised"), (2048, 64, 2, 2, 1, "constant"),
     (4096, 100, 2, 2, 1, "zeros"), (1500, 200, 2, 2, 1, "bf16like"), (2000, 128, 2, 2, 1, "negative"),
-    # rows of more than 16384 pages: a cluster of four CTAs per row (uneven parts, ties, the fall-back)
+    # rows of more than 16384 pages, small k: by the maxima of groups (ties, the fall-back)
     (20000, 300, 1, 2, 1, "normal"), (16385, 64, 1, 1, 2, "bf16like"), (65536, 4096, 1, 1, 1, "normal"),
     (65536, 256, 1, 2, 1, "quantised"), (30000, 128, 1, 2, 1, "constant"), (40000, 200, 1, 2, 1, "zeros"),
     (50000, 100, 1, 2, 1, "negative"), (65536, 256, 1, 2, 1, "outlier"), (65534, 512, 2, 4, 1, "normal"),
+    # ... large k: a cluster of four CTAs per row (uneven parts, ties, the fall-back)
+    (16385, 1366, 1, 1, 2, "normal"), (16385, 2048, 1, 2, 1, "bf16like"), (20001, 1366, 1, 2, 1, "quantised"),
+    (20001, 4096, 1, 1, 1, "constant"), (32769, 684, 2, 4, 1, "normal"), (40000, 1000, 1, 2, 1, "zeros"),
+    (50000, 700, 1, 2, 1, "negative"), (65534, 684, 2, 4, 1, "outlier"), (65534, 1500, 1, 2, 1, "needles"),
+    (65535, 1500, 1, 2, 1, "runs"), (65536, 1000, 1, 2, 1, "nan"), (65536, 4095, 1, 2, 1, "inf"),
+    (65533, 700, 9, 4, 1, "normal"),      # 36 rows: just as many clusters as find their SMs, then one more head
+    (65533, 700, 10, 4, 1, "normal"),
 ])
 def test_topk_bit_exact(da, pages, k, hk, rep, s, kind):
     g = _g(pages * 7 + k)
@@ -143,6 +150,14 @@ def test_topk_bit_exact(da, pages, k, hk, rep, s, kind):
     elif kind == "outlier":
         sc[..., 5] = 1e30                   # the row's range is useless for equal-width buckets
         sc[..., 77] = -1e30
+    elif kind == "needles":
+        sc[..., torch.randperm(pages, generator=g)[:32]] += 900.0
+    elif kind == "runs":
+        sc = torch.nn.functional.avg_pool1d(torch.randn(s, hk * rep, pages + 24, generator=g) * 150, 25, stride=1)
+    elif kind == "nan":
+        sc[..., pages // 2] = float("nan")
+    elif kind == "inf":
+        sc[..., 3], sc[..., pages - 1] = float("inf"), float("-inf")
     got = _topk(da, sc, hk, rep, k)
     want = _topk_oracle(sc, hk, rep, k)
     assert torch.equal(got, want)
@@ -805,7 +820,7 @@ def test_build_pages_bytes(da, hk, tokens, page, d, dtype, offset, extra):
 
 # ------------------------------------------------------------- selection of long rows, one CTA each ----
 
-@pytest.mark.parametrize("pages,k", [(16385, 1), (16388, 1365), (16388, 1366), (32768, 300), (32769, 300), (32772, 682), (32772, 683),
+@pytest.mark.parametrize("pages,k", [(16385, 1), (16388, 1365), (16388, 1366), (32768, 300), (32769, 300), (32772, 683), (32772, 684),
                                      (65535, 256), (65536, 682), (65537, 200), (65540, 341), (65540, 342), (131072, 100),
                                      (131075, 256)])
 @pytest.mark.parametrize("kind", ["normal", "needles", "quantised", "outlier", "nan", "inf", "falling", "runs", "runs+needles"])
