@@ -102,13 +102,15 @@ __global__ void build_pages_kernel(const T *__restrict__ k, const T *__restrict_
 // The same pass with 16 bytes per thread and load: 2 * chunks consecutive threads take one page of one head
 // (chunks = 16-byte pieces of a row), thread c the c-th piece of its key row, then value row, of every token, so that
 // a token leaves as one contiguous run of both rows and a thread sees all the keys of its channels (no exchange for
-// the summaries).  For rows of whole 16-byte pieces, at most 1 KB long, on 16-byte boundaries.  Neighbouring groups take the heads of a page, whose rows are neighbours in the prompt's keys.
+// the summaries).  For rows of whole 16-byte pieces, at most 1 KB long, on 16-byte boundaries.  Neighbouring groups take
+// the heads of a page, whose rows are neighbours in the prompt's keys.
 constexpr int kBuildThreads = 128;
 constexpr int kBuildUnroll = 4;
 constexpr int kBuildSms = 148;
 // With pages in host memory the link is the bound, and a few CTAs keep it busy: 117 MB in 2269, 2254, 2255 us with
-// 8, 24, 148 CTAs (52 GB/s; two bytes per thread and a CTA per page: 2678).  24 of them leave the prefill attention
-// its SMs when the two run side by side.
+// 8, 24, 148 CTAs (52 GB/s; two bytes per thread and a CTA per page: 2678).  A CTA here takes 10 000 registers, more than two
+// prefill CTAs leave of an SM: beside the prompt's attention each of the 24 keeps one prefill CTA off for the transfer.
+// Pages in device memory take the whole chip.
 constexpr int kBuildLinkCtas = 24;
 
 // Per element of a 32-bit word: the smaller (larger) one as it lies in memory, the one that was there first when they
@@ -195,6 +197,13 @@ build_pages_vec_kernel(const unsigned char *__restrict__ k, const unsigned char 
     }
 }
 
+static bool in_device_memory(const void *p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeDevice;
+    (void)cudaGetLastError();
+    return false;
+}
+
 template <typename T>
 static cudaError_t launch_build(const void *k, const void *v, long long tok_stride, long long head_stride,
                                 void *dram, void *summaries, void *slots, int n_kv_heads, int n_pages,
@@ -206,7 +215,7 @@ static cudaError_t launch_build(const void *k, const void *v, long long tok_stri
     if ((all & 15) == 0 && 2 * chunks <= kBuildThreads && (long long)n_pages * n_kv_heads <= 0x7fffffffll) {
         const long long groups = kBuildThreads / (2 * chunks);
         long long ctas = ((long long)n_pages * n_kv_heads + groups - 1) / groups;
-        const long long most = dram ? kBuildLinkCtas : 12 * kBuildSms;
+        const long long most = dram && !in_device_memory(dram) ? kBuildLinkCtas : 12 * kBuildSms;
         if (ctas > most) ctas = most;
         build_pages_vec_kernel<T><<<(unsigned)ctas, kBuildThreads, 0, stream>>>(
             static_cast<const unsigned char *>(k), static_cast<const unsigned char *>(v), tok_stride * E,

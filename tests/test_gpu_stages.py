@@ -818,6 +818,31 @@ def test_build_pages_bytes(da, hk, tokens, page, d, dtype, offset, extra):
     assert torch.equal(alone.cpu().view(bits), want.view(bits))
 
 
+def test_build_pages_into_device_memory_takes_the_whole_gpu(da):
+    """Pages may lie in device memory too: the few CTAs that saturate the host link would take many times as long as the
+    same bytes without them (pages, summaries and slots against summaries and slots of as many pages)."""
+    from dram_attention_b200.topk_selector import build_pages_
+    hk, n_pages, page, d = 8, 4096, 16, 128
+    k, v = (torch.randn(hk, n_pages * page, d, generator=torch.Generator(device=DEV).manual_seed(i), device=DEV).bfloat16()
+            for i in range(2))
+    pages, slots = (torch.empty(hk, n_pages, page, 2, d, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    summaries = torch.empty(hk, n_pages, 2, d, dtype=torch.bfloat16, device=DEV)
+
+    def us(dram, n_slots):
+        best = float("inf")
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            build_pages_(k, v, page, dram, summaries, slots if n_slots else None, n_slots)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 1e3)
+        return best
+
+    assert us(pages, 0) <= 2 * us(None, n_pages)
+    assert torch.equal(pages, slots)
+
+
 # ------------------------------------------------------------- selection of long rows, one CTA each ----
 
 @pytest.mark.parametrize("pages,k", [(16385, 1), (16388, 1365), (16388, 1366), (32768, 300), (32769, 300), (32772, 683), (32772, 684),
