@@ -3,19 +3,16 @@
 // merge in the same launch.
 //
 // Work unit = 16 consecutive tokens (8 KiB for head_dim 128 in 16-bit types).  A
-// unit of the slot table is one contiguous block (token-major, key then value), so
-// one untiled bulk copy (TMA) brings it into shared memory; a unit of the local
-// window is gathered row by row with small bulk copies into the same layout.  Every
-// warp owns a private ring of stages with one mbarrier each, so there is no
-// CTA-wide synchronisation in the main loop.
+// unit of the slot table is one contiguous block (token-major, key then value),
+// which bulk copies (TMA; one for a float32 unit, one per token for 16-bit types)
+// bring into shared memory; a unit of the local window is gathered row by row into
+// the same layout.  Every warp owns a private ring of stages with one mbarrier each,
+// so there is no CTA-wide synchronisation in the main loop.
 //
-// Arithmetic mapping: 8 lanes share a token (each owns D/8 channels, as two
-// chunks that make conflict-free 128-bit shared-memory reads), 4 tokens per warp
-// pass, all `rep` query heads of the KV head at once.  The dot products finish
-// with a 3-step shuffle tree; softmax is online in the log2 domain with float32
-// state; partial (m, l, acc) of the 4 token groups and the 4 warps are merged
-// through shuffles and shared memory, written to the workspace, and the last CTA
-// of a head (atomic ticket) merges the splits and writes the output.
+// The partial (m, l, acc) of a CTA's warps are merged through shared memory and
+// written to the workspace, and the last CTA of a head (atomic ticket) merges the
+// splits and writes the output.  This file has the arithmetic for float32 on CUDA
+// cores (SimtMath) and the host side; attn_mma.cu that of the 16-bit types.
 
 #include "attn_body.cuh"
 

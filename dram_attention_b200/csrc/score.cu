@@ -21,7 +21,8 @@ constexpr int kScoreWarps = kScoreThreads / 32;
 constexpr int kScoreUnroll = 4;
 
 // `started` (may be null) is recorded when every CTA of the launch has begun: a launch on another stream that
-// waits for it gets the SMs as this kernel's CTAs leave them, and never ahead of them.
+// waits for it gets the SMs as this kernel's CTAs leave them.  CUDA promises the moment as far as it can tell ("best
+// effort"): the order decides about time alone, never about results.
 template <typename... KArgs, typename... Args>
 static cudaError_t launch_scorer(void (*kernel)(KArgs...), dim3 grid, cudaStream_t stream, cudaEvent_t started, Args... args) {
     cudaLaunchConfig_t cfg = {};

@@ -17,7 +17,9 @@ class DRAMAttention(torch.nn.Module):
 
     `fused_fetch` (class attribute, default True): pages that miss the slot table are read
     from DRAM by the attention kernel itself and written through to their slots, instead of
-    by a separate gather-copy launch before it.  Results are identical either way.
+    by a separate gather-copy launch before it.  The layouts of a step (`fused_fetch`, `overlap`) select and
+    keep the same pages; their outputs agree to the rounding of the element type, since each deals the tokens to the SMs
+    in its own way.  Within a layout the same calls give the same bits.
 
     Two caches: a local window of the most recent tokens in HBM, and the prefix in
     pinned DRAM behind an LRU-managed HBM slot table.  Every generate step scores

@@ -306,7 +306,8 @@ DA_API int da_decode_attention(const void *q,
  *              head_dim); lse_out optional (n_q_tokens, n_kv_heads * rep)
  * workspace    da_decode_attention_tokens_workspace_bytes() bytes
  * One launch covers 16 / rep tokens for 16-bit types (8 / rep for float32), or 32 / rep of a longer call where the
- * workspace has room for as many rows (two or more KV heads); longer calls are several launches on `stream`.  Requires rep <= 16 (8 for float32), n_q_tokens <= local_capacity.
+ * workspace has room for as many rows (two or more KV heads); longer calls are several launches on `stream`.
+ * Requires rep <= 16 (8 for float32), n_q_tokens <= local_capacity.
  */
 DA_API size_t da_decode_attention_tokens_workspace_bytes(int n_kv_heads, int rep, int head_dim,
                         int n_q_tokens);
@@ -357,7 +358,7 @@ DA_API int da_decode_attention_fetch(const void *q,
 /*
  * da_decode_attention_fetch as two launches, so that nearly all of the attention runs BESIDE
  * the scoring, the selection and the LRU update instead of after them (same reference lines
- * as da_decode_attention_fetch; the result is the same).
+ * as da_decode_attention_fetch; the result is the same up to the order of the sums).
  *
  *   phase 1  (may run concurrently with da_score_pages / da_topk_pages / da_lru_update of the
  *            same step): appends the new key/value, attends over the local window and over
@@ -373,7 +374,7 @@ DA_API int da_decode_attention_fetch(const void *q,
  *            rows phase 1 wrote for that head are ignored.
  *   The CTA of a head that finishes LAST, whichever launch it belongs to, merges the
  *   partials, writes the output, and flips split_flip[h], which makes the front the update
- *   wrote current.  Both launches of a step must have been enqueued before the next step's
+ *   wrote current.  The sums are taken in the same order whichever it is.  Both launches of a step must have been enqueued before the next step's
  *   first one; a step is complete when both have finished.
  *
  * split_order, split_count, split_flip, split_redo   the evict_queue, front_count, split_flip and
@@ -386,7 +387,8 @@ DA_API int da_decode_attention_fetch(const void *q,
 DA_API size_t da_decode_attention_phased_workspace_bytes(int n_kv_heads, int rep, int head_dim);
 /* Default CTAs per KV head of phase 1; each fills an SM (for the sm_budget of da_topk_pages_wide). */
 DA_API int da_decode_attention_phase1_ctas(int n_kv_heads);
-/* 1 if da_decode_attention_phased accepts this shape (page_size a multiple of 16), else 0. */
+/* 1 if da_decode_attention_phased accepts this shape, else 0: page_size a multiple of 16, head_dim 64 or 128 (float32:
+ * 64 only, an SM holds too few stages of 128 channels), rep at most 16 (float32: 8). */
 DA_API int da_decode_attention_phased_supported(int n_kv_heads, int rep, int head_dim, int dtype,
                         int n_slots, int page_size, int local_capacity);
 DA_API int da_decode_attention_phased(int phase, const int32_t *split_order, const int32_t *split_count,
@@ -561,8 +563,9 @@ DA_API int da_gather_heads(const void *local, int bytes_per_rank, void *const *p
  *            DA_LAYOUT_OVERLAPPED          the two-launch attention: phase 1 on the fork's stream beside score,
  *                                          select and update, phase 2 after the update; one token
  *   fork     from da_fork_create (one per concurrent caller); needed by DA_LAYOUT_OVERLAPPED
- *   fork_before_score   non-zero: phase 1 starts once every CTA of the scorer has begun, so that it takes over
- *            the SMs as they leave them; zero: after the scorer
+ *   fork_before_score   non-zero: phase 1 starts once every CTA of the scorer has begun (as far as CUDA can tell), so
+ *            that it takes over the SMs as they leave them; zero: after the scorer
+ *   The selection, the update and phase 2 of DA_LAYOUT_OVERLAPPED are launched one priority level above `stream`'s.
  *   selection_sm_budget   0: 148 minus phase 1's CTAs
  *   peer_buffers (may be null), peer_seq, peer_rank, peer_world, peer_bytes   as da_decode_attention_push_next
  * Scores, page list and the miss list are scratch of the caller, sized for n_q_tokens.  The call works inside a stream
