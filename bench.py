@@ -62,7 +62,7 @@ FALLBACK_HBM_GBS = 6650.0
 NOMINAL_HBM_GBS = 8000.0
 # dram__bytes_read.sum + dram__bytes_write.sum of one single-launch attention at the default workload, from
 # the ncu capture summarised in profiles/decode_attention_mma_llama128k.md
-ATTN_TRAFFIC_BYTES_128K = 154.4e6
+ATTN_TRAFFIC_BYTES_128K = 154.9e6
 # the same counters for the phase-1 launch form of the default step (same profile file)
 PHASE1_TRAFFIC_BYTES_128K = 150.6e6
 

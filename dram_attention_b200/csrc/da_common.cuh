@@ -158,7 +158,8 @@ struct AheadOfStream {
             return 0;
         }();
         int own = 0;      // that of the default stream
-        if (stream != nullptr && cudaStreamGetPriority(stream, &own) != cudaSuccess) (void)cudaGetLastError();   // (the launches will say why)
+        if (stream != nullptr && cudaStreamGetPriority(stream, &own) != cudaSuccess)
+            (void)cudaGetLastError();   // (the launches will say why)
         else if (own > greatest) ahead_priority = own - 1;
     }
     ~AheadOfStream() { ahead_priority = 0; }

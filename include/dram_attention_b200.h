@@ -126,7 +126,8 @@ DA_API int da_topk_pages(const float *scores, int32_t *page_list,
 
 /*
  * The same selection with a hint on how many SMs it may count on.  Rows of 16 385 to 65 536
- * pages with a large k (above 1365, of more than 32 768 pages above 683) are split over a thread-block cluster of four CTAs (partial
+ * pages with a large k (above 1365, of more than 32 768 pages above 683) are split over a
+ * thread-block cluster of four CTAs (partial
  * histograms summed through distributed shared memory, candidates collected in one CTA) when all
  * clusters of the launch find an SM per CTA at once: n_tokens * n_kv_heads * rep * 4 <= sm_budget.  A caller
  * that runs another launch beside the selection (the first attention launch of the two-launch
@@ -374,7 +375,8 @@ DA_API int da_decode_attention_fetch(const void *q,
  *            rows phase 1 wrote for that head are ignored.
  *   The CTA of a head that finishes LAST, whichever launch it belongs to, merges the
  *   partials, writes the output, and flips split_flip[h], which makes the front the update
- *   wrote current.  The sums are taken in the same order whichever it is.  Both launches of a step must have been enqueued before the next step's
+ *   wrote current.  The sums are taken in the same order whichever it is.
+ *   Both launches of a step must have been enqueued before the next step's
  *   first one; a step is complete when both have finished.
  *
  * split_order, split_count, split_flip, split_redo   the evict_queue, front_count, split_flip and
